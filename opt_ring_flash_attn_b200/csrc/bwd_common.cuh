@@ -1,7 +1,10 @@
-// Launch parameters of the backward hop kernel and the GQA-group split that fills the last wave of CTAs.
+// Launch parameters of the backward hop kernel and the split of K/V tiles over CTAs that evens out the grid.
 #pragma once
 
 #include <cuda_runtime.h>
+#ifdef RFA_DEV
+#include <stdlib.h>
+#endif
 
 #include "common.h"
 
@@ -19,8 +22,8 @@ struct BwdParams {
   int accumulate_prev, causal;
   int q_begin;  // window (zigzag layout): only query rows >= q_begin contribute
   int kv_len;   // only keys < kv_len are processed; dK/dV rows beyond keep the previous partial sums (or zero)
-  int gsplit;      // CTAs per (kv tile, kv head): each takes G / gsplit query heads of the group
-  int reduce_out;  // 1: the epilogue adds into dkdv_out with vector reductions (gsplit > 1); 0: plain stores
+  int nsplit;      // CTAs per (kv tile, kv head): each takes an equal run of the group's query tiles
+  int reduce_out;  // 1: the epilogue adds into dkdv_out with vector reductions (nsplit > 1); 0: plain stores
   int* dq_order;   // ordered (bit-reproducible) dQ reductions: per-tile counters, cleared by the launcher; null = unordered
   int* status;
   unsigned long long* trace;
@@ -32,26 +35,58 @@ int bwd_check_args(const void* q, const void* k, const void* v, const void* dout
                    int Hkv, int D, int dtype, float softmax_scale, int accumulate_prev, int causal_diag, int q_begin,
                    int kv_len, const int* status);
 
-// Work units are CTAs, one per SM at a time.  A grid that is not close to a multiple of 148 wastes the last
-// wave, so a GQA group may be split over several CTAs whose partial dK/dV are added with vector reductions.
-// Picks the smallest split that fills the waves to >= 90 % and prepares dkdv_out for the reducing epilogue (copy of
-// the previous partial sums, or zeros).  Ordered mode never splits: three or more partial sums added by reductions
-// would arrive in a varying order.
-inline int choose_group_split(BwdParams& pr, long long base_units, cudaStream_t stream) {
+// Work units are CTAs, one per SM at a time; a CTA costs its query tiles plus a fixed share (prologue, filling and
+// draining the pipeline, epilogue: about kCtaOverhead tiles).  A grid that leaves SMs idle (fewer K/V tiles than SMs, a
+// nearly empty last wave, a diagonal block whose first K/V tiles see most of the queries) is evened out by giving each
+// K/V tile to several CTAs, whose partial dK/dV are added with vector reductions into a prepared buffer.
+// Picks the split with the shortest estimated makespan, a larger one only for a gain of 5 %; runs shorter than three
+// tiles cost more in reductions than they save (S = 256, 8 heads of 64: 14.3 us unsplit, 15.3 us in two).
+// Measured, hop kernel alone, unsplit / chosen (chosen split; the neighbours are slower):
+//   S 2048, 32/8 heads of 128, diagonal 183 / 108 us (2: 109, 3: 130);  16/2 heads, diagonal 344 / 66 (8: 66, 6: 74),
+//   full 348 / 101 (4);  B 2, S 1500, 16/4 heads of 96: 137 / 72 (3), full 140 / 109 (3);  S 1024, 32 heads: 49 (1).
+inline int choose_split(BwdParams& pr, long long base_units, int bq, cudaStream_t stream) {
+  constexpr int kSMs = 148;
+  constexpr double kCtaOverhead = 2.5;
+  constexpr double kSplitGain = 0.95;
+  constexpr int kMaxSplit = 16;
+  constexpr int kMinRun = 3;
   const int G = pr.Hq / pr.Hkv;
-  int best = 1;
-  double best_eff = 0.0;
-  // Diagonal (causal) blocks: CTAs carry unequal work and are launched heaviest first, so the tail evens out by itself
-  // once there are a few CTAs per SM; splitting only adds reductions and K/V reloads (measured 2 % slower at config 3).
-  const bool balanced_by_order = pr.causal && base_units >= 2 * 148;
-  for (int gsplit = 1; gsplit <= G && !balanced_by_order && pr.dq_order == nullptr; ++gsplit) {
-    if (G % gsplit) continue;
-    const long long units = base_units * gsplit;
-    const double eff = static_cast<double>(units) / static_cast<double>((units + 147) / 148 * 148);
-    if (eff > best_eff + 1e-9) { best_eff = eff; best = gsplit; }
-    if (eff >= 0.9) { best = gsplit; break; }
+  const int n_q = ceil_div(pr.Sq, bq);
+  const int n_kv = ceil_div(pr.kv_len, 128);
+  const double heaviest = static_cast<double>(G) * (n_q - pr.q_begin / bq);  // query tiles of the first K/V tile
+  double mean = heaviest;                                                     // of all of them
+  if (pr.causal) {
+    double sum = 0;
+    const int step = 128 / bq;
+    for (int k = 0; k < n_kv; ++k) {
+      const int first = k * step > pr.q_begin / bq ? k * step : pr.q_begin / bq;
+      sum += n_q - first;
+    }
+    mean = G * sum / n_kv;
   }
-  pr.gsplit = best;
+  // the ordered mode has counters for as many K/V tiles as there are query tiles of 128 rows
+  const bool may_split = pr.dq_order == nullptr ||
+                         static_cast<long long>(pr.Hkv) * n_kv <= static_cast<long long>(pr.Hq) * ceil_div(pr.Sq, 128);
+  int best = 1;
+  double best_t = 0;
+  for (int ns = 1; ns <= kMaxSplit && (ns == 1 || heaviest >= kMinRun * ns); ++ns) {
+    const double n = static_cast<double>(base_units) * ns;
+    const double longest = heaviest / ns + kCtaOverhead;
+    double t;
+    if (n <= kSMs) t = longest;
+    else if (!pr.causal) t = static_cast<double>((static_cast<long long>(n) + kSMs - 1) / kSMs) * longest;
+    else {
+      // heaviest first, so the tail is made of short CTAs: the mean load, plus half a short CTA
+      const double load = (mean / ns + kCtaOverhead) * n / kSMs + kCtaOverhead;
+      t = load > longest ? load : longest;
+    }
+    if (ns == 1 || t < best_t * kSplitGain) { best = ns; best_t = t; }
+    if (!may_split) break;
+  }
+#ifdef RFA_DEV
+  if (getenv("RFA_NS")) best = atoi(getenv("RFA_NS"));
+#endif
+  pr.nsplit = best;
   pr.reduce_out = best > 1 ? 1 : 0;
   // Rows of dkdv_out that the kernel does not write (keys beyond kv_len) must still hold prev (or zero): prepare the
   // whole buffer in that case too.

@@ -45,6 +45,24 @@ constexpr int kBwdPolyEvery = 0;
 namespace rfa {
 
 
+// Bounded wait of one lane until a counter in global memory has reached `target`; the whole warp gets the answer
+// (false: the CTA is aborting).
+__device__ __forceinline__ bool wait_count(const int* sem, int target, bool waiter, volatile int* abort_p) {
+  bool got = true;
+  if (waiter) {
+    const unsigned long long since = global_timer_ns();
+    uint32_t spins = 0;
+    while (ld_acquire_gpu(sem) < target) {
+      if (((++spins) & 0x3fu) == 0) {
+        if (*abort_p) { got = false; break; }
+        if (global_timer_ns() - since > kWaitLimitNs) { *abort_p = 1; got = false; break; }
+      }
+      __nanosleep(64);
+    }
+  }
+  return __all_sync(0xffffffffu, got);
+}
+
 template <int DP, int DH, int BQ, int NST>
 struct BwdCfg {
   static constexpr int kPanels = DP / 64;
@@ -111,14 +129,14 @@ __global__ void __launch_bounds__(640, 1)
   // some 20 MB instead of the whole 134 MB accumulator, which then stays in L2 between the reductions of
   // different kv tiles (kv-tile-first order re-fetched it from HBM: 4.3 GB of DRAM traffic per launch at
   // S = 8192, 32/8 heads, against 0.6 GB of algorithmic bytes).
-  int kvt, hf, gs, hkv, b;
+  int kvt, hf, part, hkv, b;
   {
     int rem = static_cast<int>(blockIdx.x);
     hf = rem % Cfg::kHalves;
     rem /= Cfg::kHalves;
     if (p.causal) {
-      gs = rem % p.gsplit;  // CTAs that share a K/V tile are adjacent (the tile stays in L2)
-      rem /= p.gsplit;
+      part = rem % p.nsplit;  // CTAs that share a K/V tile are adjacent (the tile stays in L2)
+      rem /= p.nsplit;
       hkv = rem % p.Hkv;
       rem /= p.Hkv;
       b = rem % p.B;
@@ -127,19 +145,20 @@ __global__ void __launch_bounds__(640, 1)
       const int nkvt = (p.kv_len + 127) / 128;
       kvt = rem % nkvt;
       rem /= nkvt;
-      gs = rem % p.gsplit;
-      rem /= p.gsplit;
+      part = rem % p.nsplit;
+      rem /= p.nsplit;
       hkv = rem % p.Hkv;
       b = rem / p.Hkv;
     }
   }
   const int G = p.Hq / p.Hkv;
-  const int Gc = G / p.gsplit;
   const int n0 = kvt * 128;
   const int nQtiles = (p.Sq + BQ - 1) / BQ;
   const int i_begin = max(p.causal ? (n0 / BQ) : 0, p.q_begin / BQ);
   const int nI = nQtiles - i_begin;
-  const int T_total = Gc * nI;
+  // The G * nI query tiles of the K/V tile, head-major, are dealt out to nsplit CTAs in equal runs [t0, t0 + T_total).
+  const int t0 = static_cast<int>(static_cast<long long>(G) * nI * part / p.nsplit);
+  const int T_total = static_cast<int>(static_cast<long long>(G) * nI * (part + 1) / p.nsplit) - t0;
 
   if (tid == 0) {
     abort_flag = ((smem_base & 1023u) != 0) ? 1 : 0;  // operand tiles need 1024-byte alignment
@@ -177,8 +196,8 @@ __global__ void __launch_bounds__(640, 1)
     if (lane == 0) role = (warp == 0) ? 0 : (warp == 1) ? 1 : (warp == 4) ? 2 : (warp == 8) ? 3 : (warp == 12) ? 4 : -1;
     if (role >= 0) tr.init(p.trace, p.trace_ctas, p.trace_cap, kTraceRoles, role);
   }
-  auto q_head = [&](int t) { return hkv * G + gs * Gc + t / nI; };
-  auto q_tile = [&](int t) { return i_begin + t % nI; };
+  auto q_head = [&](int t) { return hkv * G + (t0 + t) / nI; };
+  auto q_tile = [&](int t) { return i_begin + (t0 + t) % nI; };
 
   // Register budget.  The launch gives every thread 96 registers (640 x 96 = 61440, the pool the warpgroups trade
   // inside); each role changes its own allowance on entry: 4 service warps x 64, 8 elementwise warps x 128,
@@ -514,6 +533,14 @@ __global__ void __launch_bounds__(640, 1)
     }
     // ---- epilogue: group 0 writes dV, group 1 writes dK (scaled) ----
     if (ok) ok = mbar_wait_warp(&bar_final, 0, abort_p);
+    // Ordered mode with a split tile: the runs add in the order of their index (one counter per warp and tile), so that
+    // dK and dV are bit-reproducible too.  The run waited for has a lower block index: it was dispatched before.
+    int* part_sem = nullptr;
+    if (p.dq_order != nullptr && p.nsplit > 1) {
+      part_sem = p.dq_order + static_cast<size_t>(p.B) * p.Hq * nQtiles * Cfg::kHalves * 8 +
+                 (((static_cast<size_t>(b) * p.Hkv + hkv) * ((p.kv_len + 127) / 128) + kvt) * Cfg::kHalves + hf) * 8 + (warp - 4);
+      if ((ok || !run) && !wait_count(part_sem, part, lane == 0, abort_p)) ok = false;
+    }
     if (ok) {
       tc_fence_after_sync();
       const bool row_ok = kvpos < p.kv_len;
@@ -547,6 +574,11 @@ __global__ void __launch_bounds__(640, 1)
           }
         }
       }
+    }
+    if (part_sem != nullptr) {
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) red_release_gpu_add(part_sem, 1);
     }
     __syncwarp();
   } else {
@@ -599,19 +631,7 @@ __global__ void __launch_bounds__(640, 1)
         order_sem = p.dq_order +
                     ((((static_cast<size_t>(b) * p.Hq + hq) * nQtiles + q_tile(t)) * Cfg::kHalves + hf) * 2 + half) * 4 +
                     quarter;
-        bool got = true;
-        if (lane == 0 && d_ok) {
-          const unsigned long long t0 = global_timer_ns();
-          uint32_t spins = 0;
-          while (ld_acquire_gpu(order_sem) < kvt) {
-            if (((++spins) & 0x3fu) == 0) {
-              if (*abort_p) { got = false; break; }
-              if (global_timer_ns() - t0 > kWaitLimitNs) { *abort_p = 1; got = false; break; }
-            }
-            __nanosleep(64);
-          }
-        }
-        if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
+        if (!wait_count(order_sem, kvt, lane == 0 && d_ok, abort_p)) { ok = false; break; }
       }
       if (d_ok) {
         // rows beyond Sq and head-dim columns beyond D hold exact zeros (zero-filled operands, P = 0)
@@ -679,14 +699,15 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
   BwdParams pr = prm;
   const long long base_units = static_cast<long long>(ceil_div(prm.kv_len, 128)) * prm.Hkv * prm.B * Cfg::kHalves;
   {
-    const int rc2 = choose_group_split(pr, base_units, stream);
+    const int rc2 = choose_split(pr, base_units, BQ, stream);
     if (rc2 != RFA_OK) return rc2;
   }
   if (pr.dq_order != nullptr) {
-    const size_t n = static_cast<size_t>(prm.B) * prm.Hq * ceil_div(prm.Sq, BQ) * Cfg::kHalves * 8;
+    size_t n = static_cast<size_t>(prm.B) * prm.Hq * ceil_div(prm.Sq, BQ) * Cfg::kHalves * 8;
+    if (pr.nsplit > 1) n += static_cast<size_t>(prm.B) * prm.Hkv * ceil_div(prm.kv_len, 128) * Cfg::kHalves * 8;
     if (cudaMemsetAsync(pr.dq_order, 0, n * sizeof(int), stream) != cudaSuccess) { cudaGetLastError(); return RFA_ERR_CUDA; }
   }
-  const unsigned grid = static_cast<unsigned>(base_units * pr.gsplit);
+  const unsigned grid = static_cast<unsigned>(base_units * pr.nsplit);
   kern<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv, tdo, pr);
   return cuda_status(cudaGetLastError());
 }
@@ -729,7 +750,8 @@ static int bwd_q_tile(int dp) { return dp == 256 ? 64 : 128; }
 extern "C" size_t rfa_dq_order_elems(int B, int Sq, int Hq, int D) {
   const int dp = rfa::padded_head_dim(D);
   if (dp == 0 || B <= 0 || Sq <= 0 || Hq <= 0) return 0;
-  return static_cast<size_t>(B) * Hq * rfa::ceil_div(Sq, bwd_q_tile(dp)) * (dp == 256 ? 2 : 1) * 8;
+  // per query tile: the dQ counters; per K/V tile (as many as query tiles of 128): the counters of a split tile
+  return static_cast<size_t>(B) * Hq * (rfa::ceil_div(Sq, bwd_q_tile(dp)) + rfa::ceil_div(Sq, 128)) * (dp == 256 ? 2 : 1) * 8;
 }
 
 static int bwd_hop_impl(const void* q, const void* k, const void* v, const void* dout, const float* lse2,
@@ -764,7 +786,7 @@ static int bwd_hop_impl(const void* q, const void* k, const void* v, const void*
   prm.causal = causal_diag ? 1 : 0;
   prm.q_begin = q_begin;
   prm.kv_len = kv_len;
-  prm.gsplit = 1;
+  prm.nsplit = 1;
   prm.reduce_out = 0;
   prm.dq_order = dq_order;
   prm.status = status;

@@ -211,8 +211,8 @@ def backward_workspace(q: torch.Tensor, k: torch.Tensor, world_size: int,
         kv_send, kv_recv = kv[0], kv[1:]
         block_dkdv = torch.empty(2, B, S, Hkv, D, dtype=torch.float32, device=dev)
     status, status_host = _new_status(dev)
-    # counters of the ordered dQ reductions: 8 per (batch, head, query tile of 64 rows) covers every head dim
-    dq_order = torch.zeros(B * Hq * ((S + 63) // 64) * 2 * 8, dtype=torch.int32, device=dev)
+    # counters of the ordered reductions: per query tile and per K/V tile, sized for every head dim
+    dq_order = torch.zeros(B * Hq * ((S + 63) // 64 + (S + 127) // 128) * 2 * 8, dtype=torch.int32, device=dev)
     ws = BackwardWorkspace(delta, lse2, dq_acc, dkdv, block_dkdv, kv_send, kv_recv, status, dq_order, status_host,
                            comms=comms)
     _bwd_cache[owner] = (key, ws)
