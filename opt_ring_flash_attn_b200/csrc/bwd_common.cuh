@@ -11,6 +11,7 @@
 namespace rfa {
 
 struct BwdParams {
+  const void* k;  // for head dim 256, where K is also copied into tensor memory
   const float* lse2;
   const float* delta;
   float* dq_acc;

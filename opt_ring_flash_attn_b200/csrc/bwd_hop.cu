@@ -20,8 +20,13 @@
 // warpgroups (each owns half of the query columns of every tile: P^T, dS^T, then
 // the dV / dK epilogues), warps 12-19 two dQ reduction warpgroups (half of the
 // query columns each).
-// Tensor memory: [0,BQ) S^T / P^T, [BQ,2BQ) dP^T then dQ^T, then dV (DH) and dK (DH).
-// Head dim 256 runs as two CTAs per tile, each owning 128 columns of dK, dV, dQ.
+// Tensor memory: [0,BQ) S^T / P^T, [BQ,2BQ) dP^T then dQ^T, then dV (DH) and dK (DH), then what the head dim leaves room
+// for: dQ^T in columns of its own (64), K as the A operand of S^T (256).
+// Head dim 256 runs as two CTAs per tile, each owning 128 columns of dK, dV, dQ.  It was a serial chain: with K and V
+// of the full head dim in shared memory only one Q stage fitted, and every tile waited some 2100 of 4880 cycles for the
+// next Q to be loaded after dK had released the slot.  K in tensor memory frees 32 KB for a second Q stage, takes the A
+// reads of S^T (64 of 96 KB per tile) off the shared-memory port, and brings the tile to 3380 cycles: full block of B 2,
+// S 4096, 16 heads 2.56 -> 2.02 ms, diagonal 1.43 -> 1.25 ms (at 950 W; the clock drops as the tensor pipe fills).
 #include <type_traits>
 
 #include "bwd_common.cuh"
@@ -34,7 +39,7 @@ namespace rfa {
 // the 64 KB of dQ^T of a tile need >= 2048 cycles whatever issues them; unpaced, the eight reduction warps keep the
 // load/store queue full of reductions and every shared-memory or tensor-memory access of the elementwise warps
 // waits behind them.  The optimum is sharp (diagonal / full block at S = 8192, 32/8 heads: 0 ns 1.57 / 2.99 ms, 50 ns
-// 1.54 / 2.97, 100 ns 1.35 / 2.52, 200 ns 2.13 / 4.20).
+// 1.54 / 2.97, 100 ns 1.35 / 2.52, 200 ns 2.13 / 4.20).  Head dim 64 reduces through the copy engine instead.
 constexpr unsigned kRedSleepNs = 100;
 // Every n-th group of four exponentials of the P^T phase on the FMA pipe (0 = all on the special-function unit, which
 // measured best here: the phase is bound by shared-memory and load/store traffic, not by exp2).
@@ -63,21 +68,32 @@ __device__ __forceinline__ bool wait_count(const int* sem, int target, bool wait
   return __all_sync(0xffffffffu, got);
 }
 
-template <int DP, int DH, int BQ, int NST>
+template <int DP, int DH, int BQ, int NSQ, int NSO>
 struct BwdCfg {
   static constexpr int kPanels = DP / 64;
   static constexpr int kHalves = DP / DH;
-  static constexpr int kKBytes = 128 * DP * 2;
+  // Head dim 256: K is the A operand of S^T from tensor memory (64 KB, 128 columns), so that shared memory only holds the
+  // half of its columns that dQ^T needs and there is room for a second Q stage.
+  static constexpr bool kKTmem = (DP == 256);
+  static constexpr int kKSmemBytes = 128 * (kKTmem ? DH : DP) * 2;
+  static constexpr int kVBytes = 128 * DP * 2;
   static constexpr int kQBytes = BQ * DP * 2;
   static constexpr int kDSBytes = 128 * BQ * 2;
   static constexpr int kStatBytes = 2 * BQ * 4;
   static constexpr int kOffK = 0;
-  static constexpr int kOffV = kKBytes;
-  static constexpr int kOffQ = 2 * kKBytes;
-  static constexpr int kOffDO = kOffQ + NST * kQBytes;
-  static constexpr int kOffDS = kOffDO + NST * kQBytes;
+  static constexpr int kOffV = kKSmemBytes;
+  static constexpr int kOffQ = kOffV + kVBytes;
+  static constexpr int kOffDO = kOffQ + NSQ * kQBytes;
+  static constexpr int kOffDS = kOffDO + NSO * kQBytes;
   static constexpr int kOffStat = kOffDS + kDSBytes;
-  static constexpr int kSmemUsed = kOffStat + NST * kStatBytes;
+  // dQ^T staging for bulk reductions: per reduction warpgroup two buffers of half a tile (head dim 64 only, the larger
+  // head dims have no shared memory left for it).  Vector reductions from registers share the load/store queue with
+  // every shared-memory access and special-function instruction of the elementwise warps; the copy engine does not.
+  // S = 4096, 16 heads of 64, full block: paced reductions 350 us (100 ns) / 300 us (20 ns), bulk reductions 291 us.
+  static constexpr bool kStageDQ = (DP == 64);
+  static constexpr int kDQHalfBytes = BQ / 2 * DP * 4;
+  static constexpr int kOffDQ = (kOffStat + NSQ * kStatBytes + 127) / 128 * 128;
+  static constexpr int kSmemUsed = kOffDQ + (kStageDQ ? 4 * kDQHalfBytes : 0);
   // Pad to more than half of the SM's shared memory so that two CTAs never share an SM
   // (each CTA allocates the whole tensor memory).
   static constexpr int kSmemBytes = kSmemUsed < 120 * 1024 ? 120 * 1024 : kSmemUsed;
@@ -86,23 +102,28 @@ struct BwdCfg {
   static constexpr int kTmDP = BQ;
   static constexpr int kTmDV = 2 * BQ;
   static constexpr int kTmDK = 2 * BQ + DH;
-  static_assert(2 * BQ + 2 * DH <= 512, "tensor memory over budget");
+  // dQ^T has columns of its own where tensor memory has room for them (head dim 64), so that the next dP^T need not wait
+  // until it is drained; otherwise it takes over those of dP^T.
+  static constexpr bool kOwnDQ = (DP == 64);
+  static constexpr int kTmDQ = kOwnDQ ? 2 * BQ + 2 * DH : kTmDP;
+  static constexpr int kTmK = 2 * BQ + 2 * DH;
+  static_assert(2 * BQ + 2 * DH + (kOwnDQ ? BQ : 0) + (kKTmem ? DP / 2 : 0) <= 512, "tensor memory over budget");
   static_assert(kSmemBytes <= 232448 - 1024, "shared memory over budget");
 };
 
-template <int DP, int DH, int BQ, int NST, typename T>
+template <int DP, int DH, int BQ, int NSQ, int NSO, typename T>
 __global__ void __launch_bounds__(640, 1)
     bwd_hop_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                    const BwdParams p) {
-  using Cfg = BwdCfg<DP, DH, BQ, NST>;
+  using Cfg = BwdCfg<DP, DH, BQ, NSQ, NSO>;
   constexpr bool kBf16 = Pack2<T>::kIsBf16;
   constexpr int kPanelK = 128 * 128;  // bytes per panel of a 128-row tile
   constexpr int kPanelQ = BQ * 128;   // bytes per panel of a BQ-row tile
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ uint64_t bar_kv_full;
-  __shared__ uint64_t bar_q_full[NST], bar_q_empty[NST], bar_do_full[NST], bar_do_empty[NST];
+  __shared__ uint64_t bar_kv_full, bar_k_tmem;
+  __shared__ uint64_t bar_q_full[NSQ], bar_q_empty[NSQ], bar_do_full[NSO], bar_do_empty[NSO];
   __shared__ uint64_t bar_s_full, bar_p_ready, bar_dp_full, bar_ds_ready, bar_dq_full, bar_dq_drained, bar_final;
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_flag;
@@ -121,6 +142,7 @@ __global__ void __launch_bounds__(640, 1)
   const uint32_t s_stat = smem_base + Cfg::kOffStat;
   uint8_t* const stat_ptr = smem_raw + Cfg::kOffStat;
   uint8_t* const ds_ptr = smem_raw + Cfg::kOffDS;
+  uint8_t* const dq_ptr = smem_raw + Cfg::kOffDQ;
 
   // ---- tile coordinates ----
   // Diagonal (causal) blocks: kv tile first, so that the CTAs with the most visible queries start first and the tail
@@ -163,9 +185,12 @@ __global__ void __launch_bounds__(640, 1)
   if (tid == 0) {
     abort_flag = ((smem_base & 1023u) != 0) ? 1 : 0;  // operand tiles need 1024-byte alignment
     mbar_init(&bar_kv_full, 1);
-    for (int i = 0; i < NST; ++i) {
+    mbar_init(&bar_k_tmem, 256);
+    for (int i = 0; i < NSQ; ++i) {
       mbar_init(&bar_q_full[i], 1);
       mbar_init(&bar_q_empty[i], 1);
+    }
+    for (int i = 0; i < NSO; ++i) {
       mbar_init(&bar_do_full[i], 1);
       mbar_init(&bar_do_empty[i], 1);
     }
@@ -212,25 +237,28 @@ __global__ void __launch_bounds__(640, 1)
         tma_prefetch_desc(&tm_k);
         tma_prefetch_desc(&tm_v);
         tma_prefetch_desc(&tm_do);
-        mbar_expect_tx(&bar_kv_full, 2 * Cfg::kKBytes);
+        mbar_expect_tx(&bar_kv_full, Cfg::kKSmemBytes + Cfg::kVBytes);
+        constexpr int kPanelsK = Cfg::kKTmem ? DH / 64 : Cfg::kPanels;
+        const int k_col0 = Cfg::kKTmem ? hf * DH : 0;
 #pragma unroll
-        for (int pn = 0; pn < Cfg::kPanels; ++pn) {
-          tma_load_4d(s_k + pn * kPanelK, &tm_k, &bar_kv_full, pn * 64, hkv, n0, b);
+        for (int pn = 0; pn < kPanelsK; ++pn)
+          tma_load_4d(s_k + pn * kPanelK, &tm_k, &bar_kv_full, k_col0 + pn * 64, hkv, n0, b);
+#pragma unroll
+        for (int pn = 0; pn < Cfg::kPanels; ++pn)
           tma_load_4d(s_v + pn * kPanelK, &tm_v, &bar_kv_full, pn * 64, hkv, n0, b);
-        }
-        for (int t = 0; t < T_total; ++t) {
-          const int st = t % NST;
-          const uint32_t par_empty = ((t / NST) & 1) ^ 1;
-          const int hq = q_head(t);
-          const int i = q_tile(t);
-          // dO first: its slot frees earlier (after the dV product) than the Q slot (after dK).
-          if (!mbar_wait(&bar_do_empty[st], par_empty, abort_p)) break;
+        auto load_do = [&](int t, int hq, int i) {
+          const int so = t % NSO;
+          if (!mbar_wait(&bar_do_empty[so], ((t / NSO) & 1) ^ 1, abort_p)) return false;
           tr.mark(40);
-          mbar_expect_tx(&bar_do_full[st], Cfg::kQBytes);
+          mbar_expect_tx(&bar_do_full[so], Cfg::kQBytes);
 #pragma unroll
           for (int pn = 0; pn < Cfg::kPanels; ++pn)
-            tma_load_4d(s_do + st * Cfg::kQBytes + pn * kPanelQ, &tm_do, &bar_do_full[st], pn * 64, hq, i * BQ, b);
-          if (!mbar_wait(&bar_q_empty[st], par_empty, abort_p)) break;
+            tma_load_4d(s_do + so * Cfg::kQBytes + pn * kPanelQ, &tm_do, &bar_do_full[so], pn * 64, hq, i * BQ, b);
+          return true;
+        };
+        auto load_q = [&](int t, int hq, int i) {
+          const int st = t % NSQ;
+          if (!mbar_wait(&bar_q_empty[st], ((t / NSQ) & 1) ^ 1, abort_p)) return false;
           tr.mark(41);
           mbar_expect_tx(&bar_q_full[st], Cfg::kQBytes + Cfg::kStatBytes);
 #pragma unroll
@@ -239,6 +267,15 @@ __global__ void __launch_bounds__(640, 1)
           const size_t stat_off = (static_cast<size_t>(b) * p.Hq + hq) * p.Spad + static_cast<size_t>(i) * BQ;
           bulk_load_1d(s_stat + st * Cfg::kStatBytes, p.lse2 + stat_off, BQ * 4, &bar_q_full[st]);
           bulk_load_1d(s_stat + st * Cfg::kStatBytes + BQ * 4, p.delta + stat_off, BQ * 4, &bar_q_full[st]);
+          return true;
+        };
+        for (int t = 0; t < T_total; ++t) {
+          const int hq = q_head(t);
+          const int i = q_tile(t);
+          // With as many dO slots as Q slots the dO slot frees first (after the dV product, the Q slot after dK); with fewer
+          // the Q slot of tile t has been free since dK of tile t - 2.
+          const bool ok = (NSO < NSQ) ? (load_q(t, hq, i) && load_do(t, hq, i)) : (load_do(t, hq, i) && load_q(t, hq, i));
+          if (!ok) break;
         }
       }
       __syncwarp();
@@ -256,9 +293,10 @@ __global__ void __launch_bounds__(640, 1)
         const uint32_t tm_dk = tmem_base + Cfg::kTmDK;
 
         // Descriptor low words of the resident tiles; offsets below are in 16-byte units.
-        const uint32_t k_km = desc_lo_kmajor(s_k);                                   // K as K-major A (S^T)
+        const uint32_t k_km = desc_lo_kmajor(s_k);                                   // K as K-major A (S^T), unless in TMEM
+        const uint32_t tm_k = tmem_base + Cfg::kTmK;
         const uint32_t v_km = desc_lo_kmajor(s_v);                                   // V as K-major A (dP^T)
-        const uint32_t k_mn = desc_lo_mnmajor(s_k + hf * (DH / 64) * kPanelK, kPanelK);  // K^T as MN-major A (dQ^T)
+        const uint32_t k_mn = desc_lo_mnmajor(s_k + (Cfg::kKTmem ? 0 : hf * (DH / 64) * kPanelK), kPanelK);  // K^T as MN-major A (dQ^T)
         const uint32_t ds_km = desc_lo_kmajor(s_ds);                                 // dS^T as K-major A (dK)
         const uint32_t ds_mn = desc_lo_mnmajor(s_ds, kPanelK);                       // dS^T as MN-major B (dQ^T)
         auto q_km = [&](int st) { return desc_lo_kmajor(s_q + st * Cfg::kQBytes); };
@@ -275,8 +313,11 @@ __global__ void __launch_bounds__(640, 1)
           const uint32_t bq = q_km(st);
 #pragma unroll
           for (int ks = 0; ks < DP / 16; ++ks)
-            mma_ss_lo_e(tm_s, k_km + (((ks >> 2) * kPanelK + (ks & 3) * 32) >> 4),
-                      bq + (((ks >> 2) * kPanelQ + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u, el);
+            if constexpr (Cfg::kKTmem)
+              mma_ts_lo_e(tm_s, tm_k + ks * 8, bq + (((ks >> 2) * kPanelQ + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u, el);
+            else
+              mma_ss_lo_e(tm_s, k_km + (((ks >> 2) * kPanelK + (ks & 3) * 32) >> 4),
+                          bq + (((ks >> 2) * kPanelQ + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u, el);
         };
         // dP^T[128 x BQ] = V[128 x DP] * dO[BQ x DP]^T
         auto issue_dp = [&](int st) {
@@ -310,10 +351,11 @@ __global__ void __launch_bounds__(640, 1)
         auto issue_dq = [&]() {
 #pragma unroll
           for (int ks = 0; ks < 128 / 16; ++ks)
-            mma_ss_lo_e(tm_dp, k_mn + ((ks * 2048) >> 4), ds_mn + ((ks * 2048) >> 4), idesc_dq, ks > 0 ? 1u : 0u, el);
+            mma_ss_lo_e(tmem_base + Cfg::kTmDQ, k_mn + ((ks * 2048) >> 4), ds_mn + ((ks * 2048) >> 4), idesc_dq, ks > 0 ? 1u : 0u, el);
         };
 
         bool ok = mbar_wait_warp(&bar_kv_full, 0, abort_p);
+        if (ok && Cfg::kKTmem) ok = mbar_wait_warp(&bar_k_tmem, 0, abort_p);
         if (ok) ok = mbar_wait_warp(&bar_q_full[0], 0, abort_p);
         if (ok) {
           tc_fence_after_sync();
@@ -327,16 +369,19 @@ __global__ void __launch_bounds__(640, 1)
           mma_commit_e(&bar_dp_full, el);
         }
         for (int t = 0; t < T_total && ok; ++t) {
-          const int st = t % NST;
-          const int st_n = (t + 1) % NST;
-          const uint32_t par_n = ((t + 1) / NST) & 1;
+          const int st = t % NSQ;
+          const int st_n = (t + 1) % NSQ;
+          const uint32_t par_n = ((t + 1) / NSQ) & 1;
+          const int so = t % NSO;
+          const int so_n = (t + 1) % NSO;
+          const uint32_t par_on = ((t + 1) / NSO) & 1;
           const bool more = (t + 1 < T_total);
           tr.mark(10);
           if (!mbar_wait_warp(&bar_p_ready, t & 1, abort_p)) break;
           tr.mark(11);
           tc_fence_after_sync();
-          issue_dv(st, t > 0);
-          mma_commit_e(&bar_do_empty[st], el);
+          issue_dv(so, t > 0);
+          mma_commit_e(&bar_do_empty[so], el);
           // S^T of the next tile goes out now if its Q tile has landed (a non-blocking probe); otherwise it is the
           // first thing issued once dS^T is ready.
           bool s_issued = !more;
@@ -351,14 +396,30 @@ __global__ void __launch_bounds__(640, 1)
           if (!mbar_wait_warp(&bar_ds_ready, t & 1, abort_p)) break;
           tr.mark(14);
           tc_fence_after_sync();
-          if (NST >= 2 && !s_issued) {
-            // The elementwise warps have nothing to do until S^T of the next tile exists: it goes first.  (With a
-            // single Q stage the next tile can only be loaded after dK below has released the slot.)
+          if (!s_issued) {
+            // the elementwise warps have nothing to do until S^T of the next tile exists: it goes first
             if (!mbar_wait_warp(&bar_q_full[st_n], par_n, abort_p)) break;
             tc_fence_after_sync();
             issue_s(st_n);
             mma_commit_e(&bar_s_full, el);
-            s_issued = true;
+          }
+          if (Cfg::kOwnDQ) {
+            // dP^T of the next tile does not have to wait for dQ^T: the elementwise warps find it ready
+            if (more) {
+              if (!mbar_wait_warp(&bar_do_full[so_n], par_on, abort_p)) break;
+              tc_fence_after_sync();
+              issue_dp(so_n);
+              mma_commit_e(&bar_dp_full, el);
+            }
+            issue_dk(st, t > 0);
+            mma_commit_e(&bar_q_empty[st], el);
+            if (t > 0 && !mbar_wait_warp(&bar_dq_drained, (t - 1) & 1, abort_p)) break;
+            tc_fence_after_sync();
+            issue_dq();
+            mma_commit_e(&bar_dq_full, el);
+            tr.mark(15);
+            if (!more) mma_commit_e(&bar_final, el);
+            continue;
           }
           // dK before dQ^T: it releases the Q slot ~500 cycles earlier, which matters more than the reduction
           // starting earlier (a Q tile load takes 1500-3000 cycles under the L2 load of the reductions and only two
@@ -368,19 +429,13 @@ __global__ void __launch_bounds__(640, 1)
           issue_dq();
           mma_commit_e(&bar_dq_full, el);
           tr.mark(15);
-          if (!s_issued) {
-            if (!mbar_wait_warp(&bar_q_full[st_n], par_n, abort_p)) break;
-            tc_fence_after_sync();
-            issue_s(st_n);
-            mma_commit_e(&bar_s_full, el);
-          }
           if (more) {
-            if (!mbar_wait_warp(&bar_do_full[st_n], par_n, abort_p)) break;
+            if (!mbar_wait_warp(&bar_do_full[so_n], par_on, abort_p)) break;
             tr.mark(16);
             if (!mbar_wait_warp(&bar_dq_drained, t & 1, abort_p)) break;
             tr.mark(17);
             tc_fence_after_sync();
-            issue_dp(st_n);
+            issue_dp(so_n);
             mma_commit_e(&bar_dp_full, el);
             tr.mark(18);
           } else {
@@ -412,12 +467,31 @@ __global__ void __launch_bounds__(640, 1)
     const Exp2Poly exp2_poly;
     const uint64_t nscale2 = pack_f2(-p.scale_log2, -p.scale_log2);
     bool ok = run;
+    if (Cfg::kKTmem && run) {
+      // K (16 bit, two per column) into tensor memory: each thread copies half of its row from global memory, once per CTA
+      const T* krow = static_cast<const T*>(p.k) + ((static_cast<size_t>(b) * p.Skv + kvpos) * p.Hkv + hkv) * p.D;
+#pragma unroll 1
+      for (int c = 0; c < DP / 4; c += 32) {
+        uint32_t u[32];
+        const int col = cw * (DP / 2) + 2 * c;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          uint4 w = make_uint4(0, 0, 0, 0);
+          if (kvpos < p.Skv && col + k * 8 < p.D) w = *reinterpret_cast<const uint4*>(krow + col + k * 8);
+          u[4 * k + 0] = w.x; u[4 * k + 1] = w.y; u[4 * k + 2] = w.z; u[4 * k + 3] = w.w;
+        }
+        tmem_st32(tmem_base + lane_addr + Cfg::kTmK + col / 2, u);
+      }
+      tmem_st_wait();
+      tc_fence_before_sync();
+      mbar_arrive(&bar_k_tmem);
+    }
     for (int t = 0; t < T_total && ok; ++t) {
-      const int st = t % NST;
+      const int st = t % NSQ;
       const int i = q_tile(t);
       const float* lse2_s = reinterpret_cast<const float*>(stat_ptr + st * Cfg::kStatBytes) + col0;
       const float* delta_s = lse2_s + BQ;
-      if (!mbar_wait_warp(&bar_q_full[st], (t / NST) & 1, abort_p)) { ok = false; break; }
+      if (!mbar_wait_warp(&bar_q_full[st], (t / NSQ) & 1, abort_p)) { ok = false; break; }
       tr.mark(19);
       if (!mbar_wait_warp(&bar_s_full, t & 1, abort_p)) { ok = false; break; }
       tr.mark(20);
@@ -498,6 +572,8 @@ __global__ void __launch_bounds__(640, 1)
 #pragma unroll
         for (int c = 1; c < NCH; ++c) reg_fence32(r[c]);
         tr.mark(24);
+        // the products that read the previous dS^T have retired (with dQ^T in dP^T's columns, dP^T itself says so)
+        if (Cfg::kOwnDQ && t > 0 && !mbar_wait_warp(&bar_dq_full, (t - 1) & 1, abort_p)) { ok = false; break; }
 #pragma unroll
         for (int c = 0; c < NCH; ++c) {
           uint32_t w[16];
@@ -596,7 +672,7 @@ __global__ void __launch_bounds__(640, 1)
     const int d = hf * DH + drow;
     const bool d_ok = (drow < DH);
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const uint32_t a_dq = tmem_base + lane_addr + Cfg::kTmDP + half * kRedCols;
+    const uint32_t a_dq = tmem_base + lane_addr + Cfg::kTmDQ + half * kRedCols;
     // dQ accumulator layout (fp32, private): [b][hq][Spad/128 tiles][32 groups of 4 rows][DP][4].
     // Lane = head-dim index, four consecutive registers = four consecutive query rows, so one
     // 16-byte vector reduction per (lane, row group) and 512 contiguous bytes per warp instruction.
@@ -613,11 +689,13 @@ __global__ void __launch_bounds__(640, 1)
       float* base = p.dq_acc + ((static_cast<size_t>(b) * p.Hq + hq) * nQt128 + q0 / 128) * kTileElems +
                     (static_cast<size_t>((q0 % 128 + half * kRedCols) / 4) * DP + d) * 4;
       uint32_t r[NCR][32];
+      if (d_ok) {
 #pragma unroll
-      for (int c = 0; c < NCR; ++c) tmem_ld32(a_dq + c * 32, r[c]);
-      tmem_ld_wait32(r[0]);
+        for (int c = 0; c < NCR; ++c) tmem_ld32(a_dq + c * 32, r[c]);
+        tmem_ld_wait32(r[0]);
 #pragma unroll
-      for (int c = 1; c < NCR; ++c) reg_fence32(r[c]);
+        for (int c = 1; c < NCR; ++c) reg_fence32(r[c]);
+      }
       // every read of this half of dQ^T has completed: the columns may be overwritten by the next dP^T
       tc_fence_before_sync();
       mbar_arrive(&bar_dq_drained);
@@ -633,7 +711,26 @@ __global__ void __launch_bounds__(640, 1)
                     quarter;
         if (!wait_count(order_sem, kvt, lane == 0 && d_ok, abort_p)) { ok = false; break; }
       }
-      if (d_ok) {
+      if (Cfg::kStageDQ && order_sem == nullptr) {
+        if (d_ok) {
+          const int buf = t & 1;
+          float4* stage = reinterpret_cast<float4*>(dq_ptr + (half * 2 + buf) * Cfg::kDQHalfBytes) + drow;
+          if (drow == 0) bulk_wait_read<1>();  // the reduction issued two tiles ago has read this buffer
+          named_barrier(1 + half, DH);
+#pragma unroll
+          for (int c = 0; c < NCR; ++c)
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              stage[(c * 8 + k) * DP] = make_float4(__uint_as_float(r[c][4 * k + 0]) * p.scale, __uint_as_float(r[c][4 * k + 1]) * p.scale,
+                                                    __uint_as_float(r[c][4 * k + 2]) * p.scale, __uint_as_float(r[c][4 * k + 3]) * p.scale);
+          fence_proxy_async_smem();
+          named_barrier(1 + half, DH);
+          if (drow == 0) {
+            bulk_reduce_add_f32(base, smem_base + Cfg::kOffDQ + (half * 2 + buf) * Cfg::kDQHalfBytes, Cfg::kDQHalfBytes);
+            bulk_commit();
+          }
+        }
+      } else if (d_ok) {
         // rows beyond Sq and head-dim columns beyond D hold exact zeros (zero-filled operands, P = 0)
 #pragma unroll
         for (int c = 0; c < NCR; ++c) {
@@ -652,6 +749,7 @@ __global__ void __launch_bounds__(640, 1)
         }
       }
     }
+    if (Cfg::kStageDQ && drow == 0) bulk_wait<0>();
     __syncwarp();
   }
 
@@ -669,17 +767,17 @@ __global__ void __launch_bounds__(640, 1)
   }
 }
 
-template <int DP, int DH, int BQ, int NST, typename T>
+template <int DP, int DH, int BQ, int NSQ, int NSO, typename T>
 static int launch_bwd(const void* q, const void* k, const void* v, const void* dout, const BwdParams& prm, int dtype,
                       cudaStream_t stream) {
-  using Cfg = BwdCfg<DP, DH, BQ, NST>;
+  using Cfg = BwdCfg<DP, DH, BQ, NSQ, NSO>;
   CUtensorMap tq, tk, tv, tdo;
   int rc;
   if ((rc = make_tmap_bshd(&tq, q, dtype, prm.B, prm.Sq, prm.Hq, prm.D, BQ)) != RFA_OK) return rc;
   if ((rc = make_tmap_bshd(&tdo, dout, dtype, prm.B, prm.Sq, prm.Hq, prm.D, BQ)) != RFA_OK) return rc;
   if ((rc = make_tmap_bshd(&tk, k, dtype, prm.B, prm.Skv, prm.Hkv, prm.D, 128)) != RFA_OK) return rc;
   if ((rc = make_tmap_bshd(&tv, v, dtype, prm.B, prm.Skv, prm.Hkv, prm.D, 128)) != RFA_OK) return rc;
-  auto kern = bwd_hop_kernel<DP, DH, BQ, NST, T>;
+  auto kern = bwd_hop_kernel<DP, DH, BQ, NSQ, NSO, T>;
   // Function attributes belong to a device: the opt-in to large dynamic shared memory is made once per device.
   static bool attr_done[kMaxDevices] = {};
   int dev = 0;
@@ -716,9 +814,9 @@ template <typename T>
 static int dispatch_bwd(int dp, const void* q, const void* k, const void* v, const void* dout, const BwdParams& prm,
                         int dtype, cudaStream_t stream) {
   switch (dp) {
-    case 64: return launch_bwd<64, 64, 128, 2, T>(q, k, v, dout, prm, dtype, stream);
-    case 128: return launch_bwd<128, 128, 128, 2, T>(q, k, v, dout, prm, dtype, stream);
-    case 256: return launch_bwd<256, 128, 64, 1, T>(q, k, v, dout, prm, dtype, stream);
+    case 64: return launch_bwd<64, 64, 128, 2, 2, T>(q, k, v, dout, prm, dtype, stream);
+    case 128: return launch_bwd<128, 128, 128, 2, 2, T>(q, k, v, dout, prm, dtype, stream);
+    case 256: return launch_bwd<256, 128, 64, 2, 1, T>(q, k, v, dout, prm, dtype, stream);
     default: return RFA_ERR_UNSUPPORTED;
   }
 }
@@ -768,6 +866,7 @@ static int bwd_hop_impl(const void* q, const void* k, const void* v, const void*
   if (reinterpret_cast<uintptr_t>(dq_order) & 3u) return RFA_ERR_INVALID_ARG;
   const int dp = padded_head_dim(D);
   BwdParams prm;
+  prm.k = k;
   prm.lse2 = lse2;
   prm.delta = delta;
   prm.dq_acc = dq_acc;

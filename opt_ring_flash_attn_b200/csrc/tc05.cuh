@@ -470,6 +470,27 @@ __device__ __forceinline__ void red_add_v4_f32(float* gptr, float a, float b, fl
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(gptr), "f"(a), "f"(b), "f"(c), "f"(d)
                : "memory");
 }
+// Bulk reduction shared -> global: adds `bytes` of fp32 values (both addresses 16-byte aligned, size a multiple of 16).
+// The copy engine of the SM does the work; the load/store unit only sees the st.shared that filled the buffer.
+__device__ __forceinline__ void bulk_reduce_add_f32(float* gptr, uint32_t smem_src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(gptr), "r"(smem_src),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// At most N of this thread's groups still read their shared-memory source / are still outstanding.
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait() {
+  asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
+}
+// Barrier of a subset of the block's warps (id 1..15; `threads` a multiple of 32).
+__device__ __forceinline__ void named_barrier(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 // Cross-CTA counters in global memory: acquire load and release add at GPU scope.
 __device__ __forceinline__ int ld_acquire_gpu(const int* gptr) {
   int v;
