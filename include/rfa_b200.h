@@ -218,6 +218,19 @@ int rfa_bwd_dq_finalize(const float* dq_acc, void* dq, int B, int Sq, int Hq, in
 int rfa_cast_from_f32(const float* src, void* dst, size_t n, int dtype, void* stream);
 
 /*
+ * The backward pass of a shard that has no ring (world size 1): rfa_bwd_prepare, one hop of the shard on itself and the
+ * conversions to dq, dk, dv ([B,S,H,D] in dtype), in three launches.  Replaces the whole of `_ring_backward_native` at
+ * world size 1 (optimized_ring_flash_attn.py:946-1029).
+ *  delta, lse2, dq_acc  scratch as for rfa_bwd_prepare;  dkdv  scratch, fp32 [2,B,S,Hkv,D]
+ *  dq_order             NULL, or rfa_dq_order_elems(B,S,Hq,D) counters: the ordered mode of rfa_bwd_hop_ordered
+ * Inputs, scratch and results start on 16-byte boundaries.
+ */
+int rfa_bwd_local(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
+                  float* delta, float* lse2, float* dq_acc, float* dkdv, void* dq, void* dk, void* dv, int B, int S,
+                  int Hq, int Hkv, int D, int dtype, float softmax_scale, int causal, int* dq_order, int* status,
+                  void* stream);
+
+/*
  * Packs K and V ([B, Skv, Hkv, D] each, `bytes_each` bytes) into one contiguous
  * [2, B, Skv, Hkv, D] transport buffer.  Replaces `kv_send[0].copy_(k);
  * kv_send[1].copy_(v)` (optimized_ring_flash_attn.py:836-838, 974-976).

@@ -47,6 +47,7 @@ SIGNATURES = {
     "rfa_bwd_hop": (_i, [_vp] * 9 + [_i] * 7 + [_f] + [_i] * 2 + [_vp, _vp]),
     "rfa_dq_order_elems": (_sz, [_i, _i, _i, _i]),
     "rfa_bwd_hop_ordered": (_i, [_vp] * 9 + [_i] * 7 + [_f] + [_i] * 4 + [_vp, _vp, _vp]),
+    "rfa_bwd_local": (_i, [_vp] * 13 + [_i] * 6 + [_f, _i, _vp, _vp, _vp]),
     "rfa_noalloc_scratch_bytes": (_sz, []),
     "rfa_bwd_hop_noalloc": (_i, [_vp] * 9 + [_i] * 7 + [_f] + [_i] * 2 + [_vp, _vp]),
     "rfa_dkdv_accumulate": (_i, [_vp, _vp, _vp, _sz, _vp]),
@@ -204,6 +205,21 @@ def dq_order_elems(B: int, Sq: int, Hq: int, D: int) -> int:
     if n == 0:
         raise RuntimeError(f"unsupported shape for the dQ ordering counters: B={B} S={Sq} H={Hq} D={D}")
     return n
+
+
+def bwd_local(q, k, v, out, dout, lse, delta, lse2, dq_acc, dkdv, dq, dk, dv, softmax_scale: float, causal: bool, status,
+              stream=None, dq_order: Optional[torch.Tensor] = None) -> None:
+    """The backward pass of a shard without a ring (``rfa_bwd_local``): ``dq``, ``dk``, ``dv`` in the input dtype, the
+    other outputs are scratch.  ``dq_order`` as in :func:`bwd_hop`."""
+    B, S, Hq, D = q.shape
+    assert dq_order is None or (dq_order.dtype == torch.int32 and dq_order.numel() >= dq_order_elems(B, S, Hq, D))
+    with _on_device(q):
+        rc = load().rfa_bwd_local(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), delta.data_ptr(),
+            lse2.data_ptr(), dq_acc.data_ptr(), dkdv.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+            B, S, Hq, k.shape[2], D, DTYPE_CODES[q.dtype], float(softmax_scale), int(causal), _ptr(dq_order),
+            status.data_ptr(), _stream(stream, q))
+    _check(rc, "rfa_bwd_local", kernels=3)
 
 
 def bwd_hop_noalloc(q, k, v, dout, lse2, delta, dq, dkdv_prev, dkdv_out, softmax_scale: float,

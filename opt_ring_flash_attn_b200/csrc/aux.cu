@@ -85,11 +85,20 @@ __device__ __forceinline__ float dot8<__half>(const uint4& a, const uint4& b) {
   return s;
 }
 
+// Also clears up to three buffers that the backward hop adds into (16-byte vectors): a memset of its own per buffer costs
+// a launch, some 2 us of a short shard's pass.
 template <typename T>
 __global__ void __launch_bounds__(256) bwd_prepare_kernel(const T* __restrict__ out, const T* __restrict__ dout,
                                                          const float* __restrict__ lse, float* __restrict__ delta,
                                                          float* __restrict__ lse2, int B, int Sq, int Spad, int Hq,
-                                                         int D) {
+                                                         int D, const ClearList clear) {
+  {
+    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < clear.n16[c]; i += stride)
+        clear.ptr[c][i] = make_uint4(0, 0, 0, 0);
+  }
   // A row of D 16-bit values is D/8 16-byte vectors; a group of gsz lanes (gsz = 4, 8, 16 or 32, the
   // power of two >= D/8) owns one row, so a warp streams 32/gsz rows at a time with every lane loading.
   const int vec_per_row = D / 8;
@@ -123,48 +132,6 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const T* __restrict__ 
     if (in_range && gl == 0) {
       delta[stat] = real ? acc : 0.f;
       lse2[stat] = real ? lse[stat] * 1.4426950408889634f : INFINITY;
-    }
-  }
-}
-
-// dQ accumulator (fp32, tiled [b][h][tile of 128 rows][32 row groups][DP][4]) -> dq [B, Sq, Hq, D] in T.
-// One block per (b, h, tile, 64-wide slice of the head dim); transposed through shared memory so that
-// both the reads (16 B per thread, consecutive) and the writes (16 B per thread, row-contiguous) coalesce.
-template <typename T>
-__global__ void __launch_bounds__(256) dq_finalize_kernel(const float* __restrict__ acc, T* __restrict__ dq, int B,
-                                                         int Sq, int Hq, int D, int DP, int nQt) {
-  __shared__ __align__(16) T tile[128][64 + 8];
-  const int nslice = DP / 64;
-  int idx = blockIdx.x;
-  const int slice = idx % nslice; idx /= nslice;
-  const int qt = idx % nQt; idx /= nQt;
-  const int h = idx % Hq;
-  const int b = idx / Hq;
-  const float* src = acc + ((static_cast<size_t>(b) * Hq + h) * nQt + qt) * (static_cast<size_t>(128) * DP);
-  const int dl = threadIdx.x & 63;
-  const int qsub = threadIdx.x >> 6;
-#pragma unroll 2
-  for (int qg = qsub; qg < 32; qg += 4) {
-    const float4 v = *reinterpret_cast<const float4*>(src + (static_cast<size_t>(qg) * DP + slice * 64 + dl) * 4);
-    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-      tile[4 * qg + 0][dl] = __float2bfloat16_rn(v.x); tile[4 * qg + 1][dl] = __float2bfloat16_rn(v.y);
-      tile[4 * qg + 2][dl] = __float2bfloat16_rn(v.z); tile[4 * qg + 3][dl] = __float2bfloat16_rn(v.w);
-    } else {
-      tile[4 * qg + 0][dl] = __float2half_rn(v.x); tile[4 * qg + 1][dl] = __float2half_rn(v.y);
-      tile[4 * qg + 2][dl] = __float2half_rn(v.z); tile[4 * qg + 3][dl] = __float2half_rn(v.w);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int id = it * 256 + threadIdx.x;
-    const int q = id >> 3;
-    const int part = id & 7;
-    const int qg_ = qt * 128 + q;
-    const int d = slice * 64 + part * 8;
-    if (qg_ < Sq && d < D) {
-      const uint4 w = *reinterpret_cast<const uint4*>(&tile[q][part * 8]);
-      *reinterpret_cast<uint4*>(dq + ((static_cast<size_t>(b) * Sq + qg_) * Hq + h) * D + d) = w;
     }
   }
 }
@@ -204,6 +171,70 @@ struct Cvt16<__half> {
     return __half22float2(*reinterpret_cast<const __half2*>(&u));
   }
 };
+
+// dQ accumulator (fp32, tiled [b][h][tile of 128 rows][32 row groups][DP][4]) -> dq [B, Sq, Hq, D] in T.
+// One block per (b, h, tile, 64-wide slice of the head dim); transposed through shared memory so that
+// both the reads (16 B per thread, consecutive) and the writes (16 B per thread, row-contiguous) coalesce.
+// With dkdv (fp32 [2][n]) given, the blocks beyond the dQ tiles convert it to dk and dv, kCastVec vectors of 8 per block.
+constexpr int kCastVec = 1024;
+template <typename T>
+__global__ void __launch_bounds__(256) dq_finalize_kernel(const float* __restrict__ acc, T* __restrict__ dq, int B,
+                                                         int Sq, int Hq, int D, int DP, int nQt, int dq_blocks,
+                                                         const float* __restrict__ dkdv, T* __restrict__ dk,
+                                                         T* __restrict__ dv, size_t n8) {
+  if (static_cast<int>(blockIdx.x) >= dq_blocks) {
+    const size_t i0 = static_cast<size_t>(blockIdx.x - dq_blocks) * kCastVec + threadIdx.x;
+#pragma unroll
+    for (int it = 0; it < kCastVec / 256; ++it) {
+      const size_t i = i0 + it * 256;
+      if (i < 2 * n8) {
+        const float4 a = *reinterpret_cast<const float4*>(dkdv + i * 8);
+        const float4 c = *reinterpret_cast<const float4*>(dkdv + i * 8 + 4);
+        uint4 o;
+        o.x = Cvt16<T>::pack(a.x, a.y);
+        o.y = Cvt16<T>::pack(a.z, a.w);
+        o.z = Cvt16<T>::pack(c.x, c.y);
+        o.w = Cvt16<T>::pack(c.z, c.w);
+        *reinterpret_cast<uint4*>(i < n8 ? dk + i * 8 : dv + (i - n8) * 8) = o;
+      }
+    }
+    return;
+  }
+  __shared__ __align__(16) T tile[128][64 + 8];
+  const int nslice = DP / 64;
+  int idx = blockIdx.x;
+  const int slice = idx % nslice; idx /= nslice;
+  const int qt = idx % nQt; idx /= nQt;
+  const int h = idx % Hq;
+  const int b = idx / Hq;
+  const float* src = acc + ((static_cast<size_t>(b) * Hq + h) * nQt + qt) * (static_cast<size_t>(128) * DP);
+  const int dl = threadIdx.x & 63;
+  const int qsub = threadIdx.x >> 6;
+#pragma unroll 2
+  for (int qg = qsub; qg < 32; qg += 4) {
+    const float4 v = *reinterpret_cast<const float4*>(src + (static_cast<size_t>(qg) * DP + slice * 64 + dl) * 4);
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      tile[4 * qg + 0][dl] = __float2bfloat16_rn(v.x); tile[4 * qg + 1][dl] = __float2bfloat16_rn(v.y);
+      tile[4 * qg + 2][dl] = __float2bfloat16_rn(v.z); tile[4 * qg + 3][dl] = __float2bfloat16_rn(v.w);
+    } else {
+      tile[4 * qg + 0][dl] = __float2half_rn(v.x); tile[4 * qg + 1][dl] = __float2half_rn(v.y);
+      tile[4 * qg + 2][dl] = __float2half_rn(v.z); tile[4 * qg + 3][dl] = __float2half_rn(v.w);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int id = it * 256 + threadIdx.x;
+    const int q = id >> 3;
+    const int part = id & 7;
+    const int qg_ = qt * 128 + q;
+    const int d = slice * 64 + part * 8;
+    if (qg_ < Sq && d < D) {
+      const uint4 w = *reinterpret_cast<const uint4*>(&tile[q][part * 8]);
+      *reinterpret_cast<uint4*>(dq + ((static_cast<size_t>(b) * Sq + qg_) * Hq + h) * D + d) = w;
+    }
+  }
+}
 
 // out16 = round(float(prev16) + block32) over groups of 8 elements (prev may be null: out16 = round(block32)).
 // Streams 32 + 16 + 16 bytes per group: HBM-bound.
@@ -288,6 +319,46 @@ extern "C" int rfa_status_publish(const int* status, int* host_copy, void* strea
   return RFA_OK;
 }
 
+namespace rfa {
+
+int launch_bwd_prepare(const void* out, const void* dout, const float* lse, float* delta, float* lse2, int B, int Sq,
+                       int Hq, int D, int dtype, const ClearList& clear, cudaStream_t s) {
+  const int Spad = round_up(Sq, 128);
+  const long long rows = static_cast<long long>(B) * Spad * Hq;
+  const int threads = 256;
+  long long blocks = (rows + 15) / 16;  // 8 warps per block, at least two rows per warp pass
+  if (blocks > 148ll * 16) blocks = 148ll * 16;
+  if (blocks < 1) blocks = 1;
+  if (dtype == RFA_DTYPE_BF16)
+    bwd_prepare_kernel<__nv_bfloat16><<<static_cast<unsigned>(blocks), threads, 0, s>>>(
+        static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), lse, delta, lse2, B, Sq, Spad,
+        Hq, D, clear);
+  else
+    bwd_prepare_kernel<__half><<<static_cast<unsigned>(blocks), threads, 0, s>>>(
+        static_cast<const __half*>(out), static_cast<const __half*>(dout), lse, delta, lse2, B, Sq, Spad, Hq, D, clear);
+  return cuda_status(cudaGetLastError());
+}
+
+int launch_bwd_finish(const float* dq_acc, void* dq, const float* dkdv, void* dk, void* dv, int B, int Sq, int Skv, int Hq,
+                      int Hkv, int D, int dtype, cudaStream_t s) {
+  const int dp = padded_head_dim(D);
+  const int nQt = round_up(Sq, 128) / 128;
+  const unsigned dq_blocks = static_cast<unsigned>(B) * Hq * nQt * (dp / 64);
+  const size_t n8 = dkdv ? static_cast<size_t>(B) * Skv * Hkv * D / 8 : 0;
+  const unsigned grid = dq_blocks + static_cast<unsigned>((2 * n8 + kCastVec - 1) / kCastVec);
+  if (dtype == RFA_DTYPE_BF16)
+    dq_finalize_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(
+        dq_acc, static_cast<__nv_bfloat16*>(dq), B, Sq, Hq, D, dp, nQt, static_cast<int>(dq_blocks), dkdv,
+        static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), n8);
+  else
+    dq_finalize_kernel<__half><<<grid, 256, 0, s>>>(dq_acc, static_cast<__half*>(dq), B, Sq, Hq, D, dp, nQt,
+                                                    static_cast<int>(dq_blocks), dkdv, static_cast<__half*>(dk),
+                                                    static_cast<__half*>(dv), n8);
+  return cuda_status(cudaGetLastError());
+}
+
+}  // namespace rfa
+
 extern "C" int rfa_bwd_prepare(const void* out, const void* dout, const float* lse, float* delta, float* lse2,
                                float* dq_acc, int B, int Sq, int Hq, int D, int dtype, int* status, void* stream) {
   using namespace rfa;
@@ -296,27 +367,10 @@ extern "C" int rfa_bwd_prepare(const void* out, const void* dout, const float* l
   if (B <= 0 || Sq <= 0 || Hq <= 0) return RFA_ERR_INVALID_ARG;
   if (padded_head_dim(D) == 0) return RFA_ERR_UNSUPPORTED;
   if (dtype != RFA_DTYPE_BF16 && dtype != RFA_DTYPE_FP16) return RFA_ERR_UNSUPPORTED;
-  const int Spad = round_up(Sq, 128);
-  const long long rows = static_cast<long long>(B) * Spad * Hq;
-  const size_t dq_vec4 = static_cast<size_t>(B) * Hq * Spad * padded_head_dim(D) / 4;
   if (dq_acc && (reinterpret_cast<uintptr_t>(dq_acc) & 15u)) return RFA_ERR_INVALID_ARG;
-  const int threads = 256;
-  long long blocks = (rows + 15) / 16;  // 8 warps per block, at least two rows per warp pass
-  if (blocks > 148ll * 16) blocks = 148ll * 16;
-  if (blocks < 1) blocks = 1;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dq_acc && cudaMemsetAsync(dq_acc, 0, dq_vec4 * sizeof(float4), s) != cudaSuccess) {
-    cudaGetLastError();
-    return RFA_ERR_CUDA;
-  }
-  if (dtype == RFA_DTYPE_BF16)
-    bwd_prepare_kernel<__nv_bfloat16><<<static_cast<unsigned>(blocks), threads, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), lse, delta, lse2, B, Sq, Spad,
-        Hq, D);
-  else
-    bwd_prepare_kernel<__half><<<static_cast<unsigned>(blocks), threads, 0, s>>>(
-        static_cast<const __half*>(out), static_cast<const __half*>(dout), lse, delta, lse2, B, Sq, Spad, Hq, D);
-  return cuda_status(cudaGetLastError());
+  ClearList clear;
+  if (dq_acc) clear.add(dq_acc, rfa_dq_acc_elems(B, Sq, Hq, D) * sizeof(float));
+  return launch_bwd_prepare(out, dout, lse, delta, lse2, B, Sq, Hq, D, dtype, clear, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" size_t rfa_dq_acc_elems(int B, int Sq, int Hq, int D) {
@@ -329,18 +383,11 @@ extern "C" int rfa_bwd_dq_finalize(const float* dq_acc, void* dq, int B, int Sq,
                                    void* stream) {
   using namespace rfa;
   if (!dq_acc || !dq || B <= 0 || Sq <= 0 || Hq <= 0) return RFA_ERR_INVALID_ARG;
-  const int dp = padded_head_dim(D);
-  if (dp == 0) return RFA_ERR_UNSUPPORTED;
+  if (padded_head_dim(D) == 0) return RFA_ERR_UNSUPPORTED;
   if (dtype != RFA_DTYPE_BF16 && dtype != RFA_DTYPE_FP16) return RFA_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(dq_acc) & 15u) || (reinterpret_cast<uintptr_t>(dq) & 15u)) return RFA_ERR_INVALID_ARG;
-  const int nQt = round_up(Sq, 128) / 128;
-  const unsigned grid = static_cast<unsigned>(B) * Hq * nQt * (dp / 64);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == RFA_DTYPE_BF16)
-    dq_finalize_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(dq_acc, static_cast<__nv_bfloat16*>(dq), B, Sq, Hq, D, dp, nQt);
-  else
-    dq_finalize_kernel<__half><<<grid, 256, 0, s>>>(dq_acc, static_cast<__half*>(dq), B, Sq, Hq, D, dp, nQt);
-  return cuda_status(cudaGetLastError());
+  return launch_bwd_finish(dq_acc, dq, nullptr, nullptr, nullptr, B, Sq, /*Skv=*/0, Hq, /*Hkv=*/0, D, dtype,
+                           static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int rfa_dkdv_accumulate(const float* prev, const float* block, float* out, size_t n, void* stream) {

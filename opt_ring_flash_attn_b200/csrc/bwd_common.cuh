@@ -2,9 +2,6 @@
 #pragma once
 
 #include <cuda_runtime.h>
-#ifdef RFA_DEV
-#include <stdlib.h>
-#endif
 
 #include "common.h"
 
@@ -17,6 +14,8 @@ struct BwdParams {
   float* dq_acc;
   const float* dkdv_prev;
   float* dkdv_out;
+  void* dk16;  // with these given and nothing to add (no split, no partial sums): dK, dV in the input dtype instead of
+  void* dv16;  // the fp32 buffer, [B, Skv, Hkv, D] each
   int B, Sq, Skv, Hq, Hkv, D;
   int Spad;
   float scale, scale_log2;
@@ -45,7 +44,7 @@ int bwd_check_args(const void* q, const void* k, const void* v, const void* dout
 // Measured, hop kernel alone, unsplit / chosen (chosen split; the neighbours are slower):
 //   S 2048, 32/8 heads of 128, diagonal 183 / 108 us (2: 109, 3: 130);  16/2 heads, diagonal 344 / 66 (8: 66, 6: 74),
 //   full 348 / 101 (4);  B 2, S 1500, 16/4 heads of 96: 137 / 72 (3), full 140 / 109 (3);  S 1024, 32 heads: 49 (1).
-inline int choose_split(BwdParams& pr, long long base_units, int bq, cudaStream_t stream) {
+inline void choose_split(BwdParams& pr, long long base_units, int bq) {
   constexpr int kSMs = 148;
   constexpr double kCtaOverhead = 2.5;
   constexpr double kSplitGain = 0.95;
@@ -84,11 +83,12 @@ inline int choose_split(BwdParams& pr, long long base_units, int bq, cudaStream_
     if (ns == 1 || t < best_t * kSplitGain) { best = ns; best_t = t; }
     if (!may_split) break;
   }
-#ifdef RFA_DEV
-  if (getenv("RFA_NS")) best = atoi(getenv("RFA_NS"));
-#endif
   pr.nsplit = best;
   pr.reduce_out = best > 1 ? 1 : 0;
+}
+
+// Brings dkdv_out into the state the kernel expects where it adds into the buffer or leaves rows of it alone.
+inline int prepare_dkdv(const BwdParams& pr, cudaStream_t stream) {
   // Rows of dkdv_out that the kernel does not write (keys beyond kv_len) must still hold prev (or zero): prepare the
   // whole buffer in that case too.
   const bool partial_rows = pr.kv_len < pr.Skv;

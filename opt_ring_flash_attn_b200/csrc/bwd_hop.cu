@@ -623,13 +623,27 @@ __global__ void __launch_bounds__(640, 1)
       const int which = (cw == 0) ? 1 : 0;  // packed buffer: [0] = dK, [1] = dV
       const float mul = (cw == 0) ? 1.0f : p.scale;
       const uint32_t a_acc = tmem_base + lane_addr + (cw == 0 ? Cfg::kTmDV : Cfg::kTmDK);
+      T* const out16 = static_cast<T*>(cw == 0 ? p.dv16 : p.dk16);
+      const size_t base16 = ((static_cast<size_t>(b) * p.Skv + kvpos) * p.Hkv + hkv) * p.D + hf * DH;
       const size_t base = (((static_cast<size_t>(which) * p.B + b) * p.Skv + kvpos) * p.Hkv + hkv) * p.D + hf * DH;
 #pragma unroll 1
       for (int c = 0; c < DH / 32; ++c) {
         uint32_t r[32];
         tmem_ld32(a_acc + c * 32, r);
         tmem_ld_wait32(r);
-        if (row_ok) {
+        if (row_ok && out16 != nullptr) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (hf * DH + c * 32 + k * 8 < p.D) {
+              uint4 w;
+              w.x = Pack2<T>::pack(__uint_as_float(r[8 * k + 0]) * mul, __uint_as_float(r[8 * k + 1]) * mul);
+              w.y = Pack2<T>::pack(__uint_as_float(r[8 * k + 2]) * mul, __uint_as_float(r[8 * k + 3]) * mul);
+              w.z = Pack2<T>::pack(__uint_as_float(r[8 * k + 4]) * mul, __uint_as_float(r[8 * k + 5]) * mul);
+              w.w = Pack2<T>::pack(__uint_as_float(r[8 * k + 6]) * mul, __uint_as_float(r[8 * k + 7]) * mul);
+              *reinterpret_cast<uint4*>(out16 + base16 + c * 32 + k * 8) = w;
+            }
+          }
+        } else if (row_ok) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             const int d = hf * DH + c * 32 + k * 4;
@@ -794,19 +808,9 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
     if (fa.numRegs * Cfg::kThreads < 128 * 64 + 256 * 128 + 256 * 80) return RFA_ERR_UNSUPPORTED;
     attr_done[dev] = true;
   }
-  BwdParams pr = prm;
   const long long base_units = static_cast<long long>(ceil_div(prm.kv_len, 128)) * prm.Hkv * prm.B * Cfg::kHalves;
-  {
-    const int rc2 = choose_split(pr, base_units, BQ, stream);
-    if (rc2 != RFA_OK) return rc2;
-  }
-  if (pr.dq_order != nullptr) {
-    size_t n = static_cast<size_t>(prm.B) * prm.Hq * ceil_div(prm.Sq, BQ) * Cfg::kHalves * 8;
-    if (pr.nsplit > 1) n += static_cast<size_t>(prm.B) * prm.Hkv * ceil_div(prm.kv_len, 128) * Cfg::kHalves * 8;
-    if (cudaMemsetAsync(pr.dq_order, 0, n * sizeof(int), stream) != cudaSuccess) { cudaGetLastError(); return RFA_ERR_CUDA; }
-  }
-  const unsigned grid = static_cast<unsigned>(base_units * pr.nsplit);
-  kern<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv, tdo, pr);
+  const unsigned grid = static_cast<unsigned>(base_units * prm.nsplit);
+  kern<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv, tdo, prm);
   return cuda_status(cudaGetLastError());
 }
 
@@ -842,14 +846,62 @@ int rfa::bwd_check_args(const void* q, const void* k, const void* v, const void*
   return RFA_OK;
 }
 
-// Query-tile width of the backward kernel for a padded head dim (the granularity of the ordering counters).
+// Query-tile width of the backward kernel for a padded head dim (the granularity of the ordering counters), and the CTAs
+// that share the head dim of a K/V tile.
 static int bwd_q_tile(int dp) { return dp == 256 ? 64 : 128; }
+static int bwd_halves(int dp) { return dp == 256 ? 2 : 1; }
 
 extern "C" size_t rfa_dq_order_elems(int B, int Sq, int Hq, int D) {
   const int dp = rfa::padded_head_dim(D);
   if (dp == 0 || B <= 0 || Sq <= 0 || Hq <= 0) return 0;
   // per query tile: the dQ counters; per K/V tile (as many as query tiles of 128): the counters of a split tile
   return static_cast<size_t>(B) * Hq * (rfa::ceil_div(Sq, bwd_q_tile(dp)) + rfa::ceil_div(Sq, 128)) * (dp == 256 ? 2 : 1) * 8;
+}
+
+static rfa::BwdParams bwd_params(const void* k, const float* lse2, const float* delta, float* dq_acc,
+                                 const float* dkdv_prev, float* dkdv_out, int B, int Sq, int Skv, int Hq, int Hkv, int D,
+                                 float softmax_scale, int accumulate_prev, int causal_diag, int q_begin, int kv_len,
+                                 int* dq_order, int* status) {
+  using namespace rfa;
+  BwdParams prm;
+  prm.k = k;
+  prm.lse2 = lse2;
+  prm.delta = delta;
+  prm.dq_acc = dq_acc;
+  prm.dkdv_prev = dkdv_prev;
+  prm.dkdv_out = dkdv_out;
+  prm.dk16 = nullptr;
+  prm.dv16 = nullptr;
+  prm.B = B;
+  prm.Sq = Sq;
+  prm.Skv = Skv;
+  prm.Hq = Hq;
+  prm.Hkv = Hkv;
+  prm.D = D;
+  prm.Spad = round_up(Sq, 128);
+  prm.scale = softmax_scale;
+  prm.scale_log2 = softmax_scale * 1.4426950408889634f;
+  prm.accumulate_prev = accumulate_prev ? 1 : 0;
+  prm.causal = causal_diag ? 1 : 0;
+  prm.q_begin = q_begin;
+  prm.kv_len = kv_len;
+  prm.dq_order = dq_order;
+  prm.status = status;
+  prm.trace = g_trace.buf;
+  prm.trace_ctas = g_trace.ctas;
+  prm.trace_cap = g_trace.cap;
+  const int dp = padded_head_dim(D);
+  choose_split(prm, static_cast<long long>(ceil_div(kv_len, 128)) * Hkv * B * bwd_halves(dp), bwd_q_tile(dp));
+  return prm;
+}
+
+// Bytes of the ordering counters that a launch uses: per query tile, and per K/V tile where the tiles are split.
+static size_t dq_order_bytes(const rfa::BwdParams& prm) {
+  using namespace rfa;
+  const int dp = padded_head_dim(prm.D);
+  size_t n = static_cast<size_t>(prm.B) * prm.Hq * ceil_div(prm.Sq, bwd_q_tile(dp)) * bwd_halves(dp) * 8;
+  if (prm.nsplit > 1) n += static_cast<size_t>(prm.B) * prm.Hkv * ceil_div(prm.kv_len, 128) * bwd_halves(dp) * 8;
+  return n * sizeof(int);
 }
 
 static int bwd_hop_impl(const void* q, const void* k, const void* v, const void* dout, const float* lse2,
@@ -865,36 +917,58 @@ static int bwd_hop_impl(const void* q, const void* k, const void* v, const void*
   }
   if (reinterpret_cast<uintptr_t>(dq_order) & 3u) return RFA_ERR_INVALID_ARG;
   const int dp = padded_head_dim(D);
-  BwdParams prm;
-  prm.k = k;
-  prm.lse2 = lse2;
-  prm.delta = delta;
-  prm.dq_acc = dq_acc;
-  prm.dkdv_prev = dkdv_prev;
-  prm.dkdv_out = dkdv_out;
-  prm.B = B;
-  prm.Sq = Sq;
-  prm.Skv = Skv;
-  prm.Hq = Hq;
-  prm.Hkv = Hkv;
-  prm.D = D;
-  prm.Spad = round_up(Sq, 128);
-  prm.scale = softmax_scale;
-  prm.scale_log2 = softmax_scale * 1.4426950408889634f;
-  prm.accumulate_prev = accumulate_prev ? 1 : 0;
-  prm.causal = causal_diag ? 1 : 0;
-  prm.q_begin = q_begin;
-  prm.kv_len = kv_len;
-  prm.nsplit = 1;
-  prm.reduce_out = 0;
-  prm.dq_order = dq_order;
-  prm.status = status;
-  prm.trace = g_trace.buf;
-  prm.trace_ctas = g_trace.ctas;
-  prm.trace_cap = g_trace.cap;
+  const BwdParams prm = bwd_params(k, lse2, delta, dq_acc, dkdv_prev, dkdv_out, B, Sq, Skv, Hq, Hkv, D, softmax_scale,
+                                   accumulate_prev, causal_diag, q_begin, kv_len, dq_order, status);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  {
+    const int rc = prepare_dkdv(prm, s);
+    if (rc != RFA_OK) return rc;
+  }
+  if (dq_order != nullptr && cudaMemsetAsync(dq_order, 0, dq_order_bytes(prm), s) != cudaSuccess) {
+    cudaGetLastError();
+    return RFA_ERR_CUDA;
+  }
   if (dtype == RFA_DTYPE_BF16) return dispatch_bwd<__nv_bfloat16>(dp, q, k, v, dout, prm, dtype, s);
   return dispatch_bwd<__half>(dp, q, k, v, dout, prm, dtype, s);
+}
+
+// Three launches: delta/lse2 and the cleared buffers; the hop; dq (with dk, dv where the K/V tiles are split).  Unsplit
+// tiles write dk and dv in the input dtype from tensor memory, without the fp32 buffer in between.
+extern "C" int rfa_bwd_local(const void* q, const void* k, const void* v, const void* out, const void* dout,
+                             const float* lse, float* delta, float* lse2, float* dq_acc, float* dkdv, void* dq, void* dk,
+                             void* dv, int B, int S, int Hq, int Hkv, int D, int dtype, float softmax_scale, int causal,
+                             int* dq_order, int* status, void* stream) {
+  using namespace rfa;
+  if (!out || !lse || !dq_acc || !dq || !dk || !dv) return RFA_ERR_INVALID_ARG;
+  {
+    const int rc = bwd_check_args(q, k, v, dout, lse2, delta, nullptr, dkdv, B, S, S, Hq, Hkv, D, dtype, softmax_scale, 0,
+                                  causal, 0, S, status);
+    if (rc != RFA_OK) return rc;
+  }
+  if ((reinterpret_cast<uintptr_t>(dq_acc) & 15u) || (reinterpret_cast<uintptr_t>(dq) & 15u) ||
+      (reinterpret_cast<uintptr_t>(dk) & 15u) || (reinterpret_cast<uintptr_t>(dv) & 15u) ||
+      (reinterpret_cast<uintptr_t>(dq_order) & 15u) || (reinterpret_cast<uintptr_t>(out) & 15u) ||
+      (reinterpret_cast<uintptr_t>(dout) & 15u) || (reinterpret_cast<uintptr_t>(k) & 15u))
+    return RFA_ERR_INVALID_ARG;
+  const int dp = padded_head_dim(D);
+  BwdParams prm = bwd_params(k, lse2, delta, dq_acc, nullptr, dkdv, B, S, S, Hq, Hkv, D, softmax_scale, 0, causal, 0, S,
+                             dq_order, status);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  ClearList clear;
+  clear.add(dq_acc, rfa_dq_acc_elems(B, S, Hq, D) * sizeof(float));
+  if (prm.reduce_out) {
+    clear.add(dkdv, static_cast<size_t>(2) * B * S * Hkv * D * sizeof(float));
+  } else {
+    prm.dk16 = dk;
+    prm.dv16 = dv;
+  }
+  if (dq_order != nullptr) clear.add(dq_order, dq_order_bytes(prm));
+  int rc = launch_bwd_prepare(out, dout, lse, delta, lse2, B, S, Hq, D, dtype, clear, s);
+  if (rc != RFA_OK) return rc;
+  if (dtype == RFA_DTYPE_BF16) rc = dispatch_bwd<__nv_bfloat16>(dp, q, k, v, dout, prm, dtype, s);
+  else rc = dispatch_bwd<__half>(dp, q, k, v, dout, prm, dtype, s);
+  if (rc != RFA_OK) return rc;
+  return launch_bwd_finish(dq_acc, dq, prm.reduce_out ? dkdv : nullptr, dk, dv, B, S, S, Hq, Hkv, D, dtype, s);
 }
 
 extern "C" int rfa_bwd_hop_window(const void* q, const void* k, const void* v, const void* dout, const float* lse2,

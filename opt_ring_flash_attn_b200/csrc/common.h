@@ -40,6 +40,24 @@ struct TraceCfg {
 extern TraceCfg g_trace;
 constexpr int kTraceRoles = 5;
 
+// Buffers the backward's first kernel clears (16-byte aligned, sizes multiples of 16 bytes).
+struct ClearList {
+  uint4* ptr[3] = {nullptr, nullptr, nullptr};
+  size_t n16[3] = {0, 0, 0};
+  int n = 0;
+  void add(void* p, size_t bytes) {
+    ptr[n] = static_cast<uint4*>(p);
+    n16[n] = bytes / 16;
+    ++n;
+  }
+};
+// delta and lse2 from out, dout, lse; clears the listed buffers.
+int launch_bwd_prepare(const void* out, const void* dout, const float* lse, float* delta, float* lse2, int B, int Sq,
+                       int Hq, int D, int dtype, const ClearList& clear, cudaStream_t stream);
+// dq from its fp32 accumulator and, where dkdv (fp32 [2][B,Skv,Hkv,D]) is given, dk and dv from it, in one launch.
+int launch_bwd_finish(const float* dq_acc, void* dq, const float* dkdv, void* dk, void* dv, int B, int Sq, int Skv, int Hq,
+                      int Hkv, int D, int dtype, cudaStream_t stream);
+
 // Translates a CUDA runtime error into an ABI error code (and clears it).
 inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? RFA_OK : RFA_ERR_CUDA; }
 

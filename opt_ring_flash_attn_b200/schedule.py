@@ -208,12 +208,17 @@ def ring_backward(group, dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v
     wire16 = ws.dkdv[0].dtype != torch.float32
     order = {"dq_order": ws.dq_order} if deterministic else {}
     dout = dout.contiguous()
-    kn.bwd_prepare(out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.status)
-
     dq = torch.empty_like(q)
     dk = torch.empty_like(k)
     dv = torch.empty_like(v)
+    if W == 1 and hasattr(kn, "bwd_local"):
+        # nothing happens between the kernels: one call enqueues them all
+        kn.bwd_local(q, k, v, out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.dkdv[0], dq, dk, dv, softmax_scale,
+                     causal, ws.status, **order)
+        workspace.publish_status(ws, "ring_flash_attn backward")
+        return dq, dk, dv
 
+    kn.bwd_prepare(out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.status)
     if W == 1:
         buf = ws.dkdv[0]
         kn.bwd_hop(q, k, v, dout, ws.lse2, ws.delta, ws.dq_acc, None, buf, softmax_scale, False, causal, ws.status,
