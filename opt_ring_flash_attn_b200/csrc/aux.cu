@@ -172,7 +172,7 @@ struct Cvt16<__half> {
   }
 };
 
-// dQ accumulator (fp32, tiled [b][h][tile of 128 rows][32 row groups][DP][4]) -> dq [B, Sq, Hq, D] in T.
+// dQ accumulator (fp32, tiled [b][h][tile of 128 rows][DP/32][32 row groups][32][4]) -> dq [B, Sq, Hq, D] in T.
 // One block per (b, h, tile, 64-wide slice of the head dim); transposed through shared memory so that
 // both the reads (16 B per thread, consecutive) and the writes (16 B per thread, row-contiguous) coalesce.
 // With dkdv (fp32 [2][n]) given, the blocks beyond the dQ tiles convert it to dk and dv, kCastVec vectors of 8 per block.
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(256) dq_finalize_kernel(const float* __restric
   const int qsub = threadIdx.x >> 6;
 #pragma unroll 2
   for (int qg = qsub; qg < 32; qg += 4) {
-    const float4 v = *reinterpret_cast<const float4*>(src + (static_cast<size_t>(qg) * DP + slice * 64 + dl) * 4);
+    const float4 v = *reinterpret_cast<const float4*>(src + ((slice * 2 + dl / 32) * 32 + qg) * 128 + dl % 32 * 4);
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
       tile[4 * qg + 0][dl] = __float2bfloat16_rn(v.x); tile[4 * qg + 1][dl] = __float2bfloat16_rn(v.y);
       tile[4 * qg + 2][dl] = __float2bfloat16_rn(v.z); tile[4 * qg + 3][dl] = __float2bfloat16_rn(v.w);

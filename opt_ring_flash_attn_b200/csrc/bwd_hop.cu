@@ -8,7 +8,7 @@
 //   dV  += P^T dO               (P^T from tensor memory, dO MN-major)
 //   dK  += dS^T Q               (dS^T from shared memory, Q MN-major)
 //   dQ^T = K^T dS^T             (both MN-major), reduced into the fp32 dQ
-//                                accumulator in global memory with red.add.f32
+//                                accumulator in global memory
 // The epilogue adds the partial dK/dV that arrived from the previous rank and
 // writes the packed fp32 buffer that travels on.  This one kernel covers the
 // reference's `_bwd_dq_kernel` (optimized_ring_flash_attn.py:672-735),
@@ -35,11 +35,11 @@
 
 namespace rfa {
 
-// Pause (ns) a reduction warp takes after each vector reduction.  An SM can push 32 B per clock towards the L2, so
-// the 64 KB of dQ^T of a tile need >= 2048 cycles whatever issues them; unpaced, the eight reduction warps keep the
-// load/store queue full of reductions and every shared-memory or tensor-memory access of the elementwise warps
-// waits behind them.  The optimum is sharp (diagonal / full block at S = 8192, 32/8 heads: 0 ns 1.57 / 2.99 ms, 50 ns
-// 1.54 / 2.97, 100 ns 1.35 / 2.52, 200 ns 2.13 / 4.20).  Head dim 64 reduces through the copy engine instead.
+// Pause (ns) a reduction warp takes after each vector reduction (head dim 256 and the ordered mode; elsewhere the copy
+// engine reduces).  An SM can push 32 B per clock towards the L2; unpaced, the eight reduction warps keep the load/store
+// queue full of reductions and every shared-memory or tensor-memory access of the elementwise warps waits behind them.
+// The optimum is sharp (head dim 128, S = 8192, 32/8 heads, diagonal / full block: 0 ns 1.57 / 2.99 ms, 50 ns 1.54 / 2.97,
+// 100 ns 1.35 / 2.52, 200 ns 2.13 / 4.20).
 constexpr unsigned kRedSleepNs = 100;
 // Every n-th group of four exponentials of the P^T phase on the FMA pipe (0 = all on the special-function unit, which
 // measured best here: the phase is bound by shared-memory and load/store traffic, not by exp2).
@@ -86,14 +86,19 @@ struct BwdCfg {
   static constexpr int kOffDO = kOffQ + NSQ * kQBytes;
   static constexpr int kOffDS = kOffDO + NSO * kQBytes;
   static constexpr int kOffStat = kOffDS + kDSBytes;
-  // dQ^T staging for bulk reductions: per reduction warpgroup two buffers of half a tile (head dim 64 only, the larger
-  // head dims have no shared memory left for it).  Vector reductions from registers share the load/store queue with
-  // every shared-memory access and special-function instruction of the elementwise warps; the copy engine does not.
-  // S = 4096, 16 heads of 64, full block: paced reductions 350 us (100 ns) / 300 us (20 ns), bulk reductions 291 us.
-  static constexpr bool kStageDQ = (DP == 64);
-  static constexpr int kDQHalfBytes = BQ / 2 * DP * 4;
+  // dQ^T staging for bulk reductions (head dims up to 128): per reduction warp two buffers of kDQGroups row groups.  Vector
+  // reductions from registers share the load/store queue with every shared-memory access and special-function instruction
+  // of the elementwise warps; the copy engine does not.  S 4096, 16 heads of 64, full block: vector reductions 350 us
+  // (paced 100 ns) / 300 us (20 ns), bulk reductions 291.  At head dim 128 the 32 KB come from the second dO stage (dO of
+  // the next tile is wanted after dQ^T has been drained, some 2500 cycles after dV released the slot).  Steady state, which
+  // is power-limited at 950 W (S 8192, 32/8 heads, diagonal / full): 1.62 / 3.25 ms with paced vector reductions,
+  // 1.51 / 2.93 with bulk ones; 1 KB instead of 2 KB per reduction costs 4 %.
+  static constexpr bool kStageDQ = (DP <= 128);
+  static constexpr int kDQGroups = (DP == 64) ? BQ / 8 : 4;      // row groups (of 4 query rows) per bulk reduction
+  static constexpr int kDQBufBytes = kDQGroups * 512;            // one warp: 32 lanes x 16 bytes per row group
+  static constexpr int kDQWarps = 2 * (DP < 128 ? DP : 128) / 32;
   static constexpr int kOffDQ = (kOffStat + NSQ * kStatBytes + 127) / 128 * 128;
-  static constexpr int kSmemUsed = kOffDQ + (kStageDQ ? 4 * kDQHalfBytes : 0);
+  static constexpr int kSmemUsed = kOffDQ + (kStageDQ ? kDQWarps * 2 * kDQBufBytes : 0);
   // Pad to more than half of the SM's shared memory so that two CTAs never share an SM
   // (each CTA allocates the whole tensor memory).
   static constexpr int kSmemBytes = kSmemUsed < 120 * 1024 ? 120 * 1024 : kSmemUsed;
@@ -687,9 +692,9 @@ __global__ void __launch_bounds__(640, 1)
     const bool d_ok = (drow < DH);
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t a_dq = tmem_base + lane_addr + Cfg::kTmDQ + half * kRedCols;
-    // dQ accumulator layout (fp32, private): [b][hq][Spad/128 tiles][32 groups of 4 rows][DP][4].
-    // Lane = head-dim index, four consecutive registers = four consecutive query rows, so one
-    // 16-byte vector reduction per (lane, row group) and 512 contiguous bytes per warp instruction.
+    // dQ accumulator layout (fp32, private): [b][hq][Spad/128 tiles][DP/32][32 groups of 4 rows][32][4].  Lane = head-dim
+    // index, four consecutive registers = four consecutive query rows: 512 contiguous bytes per warp and row group, and
+    // what a warp adds for a tile is one contiguous run.
     constexpr size_t kTileElems = static_cast<size_t>(128) * DP;
     const int nQt128 = p.Spad / 128;
     bool ok = run;
@@ -701,7 +706,7 @@ __global__ void __launch_bounds__(640, 1)
       tr.mark(30);
       tc_fence_after_sync();
       float* base = p.dq_acc + ((static_cast<size_t>(b) * p.Hq + hq) * nQt128 + q0 / 128) * kTileElems +
-                    (static_cast<size_t>((q0 % 128 + half * kRedCols) / 4) * DP + d) * 4;
+                    (d / 32) * 4096 + (q0 % 128 + half * kRedCols) / 4 * 128;  // of the warp's 32 head-dim columns
       uint32_t r[NCR][32];
       if (d_ok) {
 #pragma unroll
@@ -727,22 +732,28 @@ __global__ void __launch_bounds__(640, 1)
       }
       if (Cfg::kStageDQ && order_sem == nullptr) {
         if (d_ok) {
-          const int buf = t & 1;
-          float4* stage = reinterpret_cast<float4*>(dq_ptr + (half * 2 + buf) * Cfg::kDQHalfBytes) + drow;
-          if (drow == 0) bulk_wait_read<1>();  // the reduction issued two tiles ago has read this buffer
-          named_barrier(1 + half, DH);
+          constexpr int kChunks = kRedCols / 4 / Cfg::kDQGroups;
+          const uint32_t wbuf = ((half * (Cfg::kDQWarps / 2) + quarter) * 2) * Cfg::kDQBufBytes;
+          static_for<0, kChunks>([&](auto ck_) {
+            constexpr int ck = decltype(ck_)::value;
+            const uint32_t buf = wbuf + ((kChunks % 2 == 0) ? (ck & 1) : (t & 1)) * Cfg::kDQBufBytes;
+            float4* stage = reinterpret_cast<float4*>(dq_ptr + buf) + lane;
+            if (lane == 0) bulk_wait_read<1>();  // the reduction before the last one has read this buffer
+            __syncwarp();
 #pragma unroll
-          for (int c = 0; c < NCR; ++c)
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-              stage[(c * 8 + k) * DP] = make_float4(__uint_as_float(r[c][4 * k + 0]) * p.scale, __uint_as_float(r[c][4 * k + 1]) * p.scale,
-                                                    __uint_as_float(r[c][4 * k + 2]) * p.scale, __uint_as_float(r[c][4 * k + 3]) * p.scale);
-          fence_proxy_async_smem();
-          named_barrier(1 + half, DH);
-          if (drow == 0) {
-            bulk_reduce_add_f32(base, smem_base + Cfg::kOffDQ + (half * 2 + buf) * Cfg::kDQHalfBytes, Cfg::kDQHalfBytes);
-            bulk_commit();
-          }
+            for (int k = 0; k < Cfg::kDQGroups; ++k) {
+              constexpr int g0 = ck * Cfg::kDQGroups;
+              const uint32_t* v = &r[(g0 + k) / 8][((g0 + k) % 8) * 4];
+              stage[k * 32] = make_float4(__uint_as_float(v[0]) * p.scale, __uint_as_float(v[1]) * p.scale,
+                                          __uint_as_float(v[2]) * p.scale, __uint_as_float(v[3]) * p.scale);
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              bulk_reduce_add_f32(base + ck * Cfg::kDQGroups * 128, smem_base + Cfg::kOffDQ + buf, Cfg::kDQBufBytes);
+              bulk_commit();
+            }
+          });
         }
       } else if (d_ok) {
         // rows beyond Sq and head-dim columns beyond D hold exact zeros (zero-filled operands, P = 0)
@@ -750,7 +761,7 @@ __global__ void __launch_bounds__(640, 1)
         for (int c = 0; c < NCR; ++c) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
-            red_add_v4_f32(base + static_cast<size_t>(c * 8 + k) * DP * 4, __uint_as_float(r[c][4 * k + 0]) * p.scale,
+            red_add_v4_f32(base + (c * 8 + k) * 128 + lane * 4, __uint_as_float(r[c][4 * k + 0]) * p.scale,
                            __uint_as_float(r[c][4 * k + 1]) * p.scale, __uint_as_float(r[c][4 * k + 2]) * p.scale,
                            __uint_as_float(r[c][4 * k + 3]) * p.scale);
             if (kRedSleepNs > 0) __nanosleep(kRedSleepNs);
@@ -763,7 +774,7 @@ __global__ void __launch_bounds__(640, 1)
         }
       }
     }
-    if (Cfg::kStageDQ && drow == 0) bulk_wait<0>();
+    if (Cfg::kStageDQ && lane == 0) bulk_wait<0>();
     __syncwarp();
   }
 
@@ -819,7 +830,7 @@ static int dispatch_bwd(int dp, const void* q, const void* k, const void* v, con
                         int dtype, cudaStream_t stream) {
   switch (dp) {
     case 64: return launch_bwd<64, 64, 128, 2, 2, T>(q, k, v, dout, prm, dtype, stream);
-    case 128: return launch_bwd<128, 128, 128, 2, 2, T>(q, k, v, dout, prm, dtype, stream);
+    case 128: return launch_bwd<128, 128, 128, 2, 1, T>(q, k, v, dout, prm, dtype, stream);
     case 256: return launch_bwd<256, 128, 64, 2, 1, T>(q, k, v, dout, prm, dtype, stream);
     default: return RFA_ERR_UNSUPPORTED;
   }
