@@ -116,7 +116,7 @@ struct BwdCfg {
   static_assert(kSmemBytes <= 232448 - 1024, "shared memory over budget");
 };
 
-template <int DP, int DH, int BQ, int NSQ, int NSO, typename T>
+template <int DP, int DH, int BQ, int NSQ, int NSO, typename T, bool kTrace>
 __global__ void __launch_bounds__(640, 1)
     bwd_hop_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(640, 1)
   volatile int* abort_p = &abort_flag;
   const bool run = (abort_flag == 0) && (T_total > 0);
 
-  Tracer tr;
+  Tracer<kTrace> tr;
   {
     int role = -1;
     // traced roles: producer, issuer, one warp of each elementwise group, one reduction warp
@@ -802,12 +802,13 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
   if ((rc = make_tmap_bshd(&tdo, dout, dtype, prm.B, prm.Sq, prm.Hq, prm.D, BQ)) != RFA_OK) return rc;
   if ((rc = make_tmap_bshd(&tk, k, dtype, prm.B, prm.Skv, prm.Hkv, prm.D, 128)) != RFA_OK) return rc;
   if ((rc = make_tmap_bshd(&tv, v, dtype, prm.B, prm.Skv, prm.Hkv, prm.D, 128)) != RFA_OK) return rc;
-  auto kern = bwd_hop_kernel<DP, DH, BQ, NSQ, NSO, T>;
+  auto kern = prm.trace != nullptr ? bwd_hop_kernel<DP, DH, BQ, NSQ, NSO, T, true> : bwd_hop_kernel<DP, DH, BQ, NSQ, NSO, T, false>;
   // Function attributes belong to a device: the opt-in to large dynamic shared memory is made once per device.
-  static bool attr_done[kMaxDevices] = {};
+  static bool attr_done[2][kMaxDevices] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) { cudaGetLastError(); return RFA_ERR_CUDA; }
-  if (!attr_done[dev]) {
+  const int traced = prm.trace != nullptr;
+  if (!attr_done[traced][dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
     if (e != cudaSuccess) { cudaGetLastError(); return RFA_ERR_CUDA; }
     // The kernel trades registers between its warpgroups inside the pool the launch allocates (threads x registers
@@ -817,7 +818,7 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
     e = cudaFuncGetAttributes(&fa, kern);
     if (e != cudaSuccess) { cudaGetLastError(); return RFA_ERR_CUDA; }
     if (fa.numRegs * Cfg::kThreads < 128 * 64 + 256 * 128 + 256 * 80) return RFA_ERR_UNSUPPORTED;
-    attr_done[dev] = true;
+    attr_done[traced][dev] = true;
   }
   const long long base_units = static_cast<long long>(ceil_div(prm.kv_len, 128)) * prm.Hkv * prm.B * Cfg::kHalves;
   const unsigned grid = static_cast<unsigned>(base_units * prm.nsplit);

@@ -85,7 +85,7 @@ __device__ __forceinline__ void issue_pv(uint32_t o_tmem, uint32_t p_tmem, uint3
   });
 }
 
-template <int DP, int BN, int NQ, int NS, typename T>
+template <int DP, int BN, int NQ, int NS, typename T, bool kTrace>
 __global__ void __launch_bounds__(128 + NQ * 128, 1)
     fwd_hop_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_holder;
   volatile int* abort_p = &abort_flag;
-  Tracer tr;
+  Tracer<kTrace> tr;
   {
     int role = -1;
     if (lane == 0) role = (warp == 0) ? 0 : (warp == 1) ? 1 : (warp == 4) ? 2 : (warp == 8) ? 3 : -1;
@@ -540,15 +540,16 @@ static int launch_fwd(const void* q, const void* k, const void* v, const FwdPara
   if ((rc = make_tmap_bshd(&tq, q, dtype, prm.B, prm.Sq, prm.Hq, prm.D, 128)) != RFA_OK) return rc;
   if ((rc = make_tmap_bshd(&tk, k, dtype, prm.B, prm.Skv, prm.Hkv, prm.D, BN)) != RFA_OK) return rc;
   if ((rc = make_tmap_bshd(&tv, v, dtype, prm.B, prm.Skv, prm.Hkv, prm.D, BN)) != RFA_OK) return rc;
-  auto kern = fwd_hop_kernel<DP, BN, NQ, NS, T>;
-  // Function attributes belong to a device: one flag per instantiation and device.
-  static bool attr_done[kMaxDevices] = {};
+  auto kern = prm.trace != nullptr ? fwd_hop_kernel<DP, BN, NQ, NS, T, true> : fwd_hop_kernel<DP, BN, NQ, NS, T, false>;
+  // Function attributes belong to a device: one flag per instantiation (traced or not) and device.
+  static bool attr_done[2][kMaxDevices] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) { cudaGetLastError(); return RFA_ERR_CUDA; }
-  if (!attr_done[dev]) {
+  const int traced = prm.trace != nullptr;
+  if (!attr_done[traced][dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
     if (e != cudaSuccess) { cudaGetLastError(); return RFA_ERR_CUDA; }
-    attr_done[dev] = true;
+    attr_done[traced][dev] = true;
   }
   const int nQs = (prm.nQt - prm.q_begin / 128 + NQ - 1) / NQ;
   const unsigned grid = static_cast<unsigned>(nQs) * prm.Hq * prm.B;
