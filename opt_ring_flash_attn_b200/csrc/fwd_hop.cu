@@ -55,6 +55,9 @@ struct FwdCfg {
   static constexpr int kSmemTiles = NQ * kQBytes + kSlots * kKVBytes;
   static constexpr int kSmemBytes = kSmemTiles + 1024;  // slack for 1024-byte alignment
   static constexpr int kThreads = 128 + NQ * 128;
+  static constexpr int kServiceRegs = 72, kSoftmaxRegs = 216;  // per thread, two-tile variants
+  static constexpr int kPoolRegs = 128 * kServiceRegs + NQ * 128 * kSoftmaxRegs;
+  static_assert(NQ == 1 || kPoolRegs <= kThreads * 168, "register allowances exceed what the launch allocates");
   static constexpr int kTmO = 0;
   static constexpr int kTmS = NQ * DP;
   static_assert(kTmS + NQ * NS * BN <= 512, "tensor memory over budget");
@@ -171,141 +174,151 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
     if (role >= 0) tr.init(p.trace, p.trace_ctas, p.trace_cap, kTraceRoles, role);
   }
 
-  if (warp == 0) {
-    // =========================== TMA producer ===========================
-    if (lane == 0) {
-      tma_prefetch_desc(&tm_q);
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
-      int nvalid = 0;
+  // Register budget of the two-tile variants: the launch gives 384 x 168; the service warps pass theirs on, so that a
+  // softmax thread holds its 128 scores without spilling (S 4096, 16 heads of 64: diagonal 61.2 -> 59.4 us, full
+  // 112.8 -> 110.0; S 2048, 32/8 heads of 128: 44.8 -> 43.0, 75.6 -> 73.3; with 56 / 224 full blocks stay at 112.3 and 74.6).
+  // The raise waits until the other warps have lowered theirs, so the sum must fit the pool.
+  if (warp < 4) {
+    if constexpr (NQ == 2) setmaxnreg_dec<Cfg::kServiceRegs>();
+    if (warp == 0) {
+      // =========================== TMA producer ===========================
+      if (lane == 0) {
+        tma_prefetch_desc(&tm_q);
+        tma_prefetch_desc(&tm_k);
+        tma_prefetch_desc(&tm_v);
+        int nvalid = 0;
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) nvalid += (ntile[q] > 0) ? 1 : 0;
-      mbar_expect_tx(&bar_q_full, static_cast<uint32_t>(nvalid) * Cfg::kQBytes);
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        if (ntile[q] > 0) {
-#pragma unroll
-          for (int pn = 0; pn < Cfg::kPanels; ++pn)
-            tma_load_4d(s_q + q * Cfg::kQBytes + pn * (128 * 128), &tm_q, &bar_q_full, pn * 64, h, m0[q], b);
-        }
-      }
-      bool ok = true;
-      for (int j = 0; j < nmax && ok; ++j) {
-#pragma unroll
-        for (int which = 0; which < 2; ++which) {
-          const int u = 2 * j + which;
-          const int slot = u % kSlots;
-          const int round = u / kSlots;
-          if (!mbar_wait(&bar_kv_empty[slot], (round & 1) ^ 1, abort_p)) {
-            ok = false;
-            break;
-          }
-          tr.mark(40 + which);
-          mbar_expect_tx(&bar_kv_full[slot], Cfg::kKVBytes);
-#pragma unroll
-          for (int pn = 0; pn < Cfg::kPanels; ++pn)
-            tma_load_4d(s_kv + slot * Cfg::kKVBytes + pn * (BN * 128), which ? &tm_v : &tm_k, &bar_kv_full[slot],
-                        pn * 64, hkv, j * BN, b);
-        }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // =========================== MMA issuer ===========================
-    // The whole warp runs this loop converged; the elected lane issues.  A commit makes its mbarrier track every MMA
-    // issued before it, so the arrival on bar_s_full for tile j+1 also tells the softmax warps that O += P_j V_j has
-    // retired; bar_pv_done is only needed after the last tile.
-    {
-      const uint32_t el = elect_one();
-      constexpr uint32_t idesc_qk = make_idesc(128, BN, kBf16, false, false);
-      constexpr uint32_t idesc_pv = make_idesc(128, DP, kBf16, false, true);
-      auto slot_of = [&](int u) { return u % kSlots; };
-      auto par_of = [&](int u) { return static_cast<uint32_t>((u / kSlots) & 1); };
-      // descriptor low words of the operand tiles (K: K-major, V: MN-major, Q: K-major)
-      auto k_lo = [&](int u) { return desc_lo_kmajor(s_kv + slot_of(u) * Cfg::kKVBytes); };
-      auto v_lo = [&](int u) { return desc_lo_mnmajor(s_kv + slot_of(u) * Cfg::kKVBytes, BN * 128); };
-      uint32_t q_lo[NQ];
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) q_lo[q] = desc_lo_kmajor(s_q + q * Cfg::kQBytes);
-      auto s_tm = [&](int q, int sb) { return tmem_base + Cfg::kTmS + (q * NS + sb) * BN; };
-      auto o_tm = [&](int q) { return tmem_base + Cfg::kTmO + q * DP; };
-      bool ok = nmax > 0;
-      if (ok) ok = mbar_wait_warp(&bar_q_full, 0, abort_p);
-      if (ok) ok = mbar_wait_warp(&bar_kv_full[slot_of(0)], par_of(0), abort_p);
-      if (ok) {
-        tc_fence_after_sync();
+        for (int q = 0; q < NQ; ++q) nvalid += (ntile[q] > 0) ? 1 : 0;
+        mbar_expect_tx(&bar_q_full, static_cast<uint32_t>(nvalid) * Cfg::kQBytes);
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
           if (ntile[q] > 0) {
-            issue_qk<DP, BN>(s_tm(q, 0), q_lo[q], k_lo(0), idesc_qk, el);
-            mma_commit_e(&bar_s_full[q * NS + 0], el);
-          }
-        }
-        mma_commit_e(&bar_kv_empty[slot_of(0)], el);
-      }
-      for (int j = 0; j < nmax && ok; ++j) {
-        if (NS == 2) {
-          // Score buffer (j+1)&1 is free: P_{j-1} was consumed by the PV issued last iteration.
-          if (j + 1 < ntile[0]) {
-            const int uk = 2 * (j + 1);
-            if (!mbar_wait_warp(&bar_kv_full[slot_of(uk)], par_of(uk), abort_p)) { ok = false; break; }
-            tc_fence_after_sync();
-            issue_qk<DP, BN>(s_tm(0, (j + 1) & 1), q_lo[0], k_lo(uk), idesc_qk, el);
-            mma_commit_e(&bar_s_full[(j + 1) & 1], el);
-            mma_commit_e(&bar_kv_empty[slot_of(uk)], el);
-          }
-        }
-        const int uv = 2 * j + 1;
-        tr.mark(9);
-        if (!mbar_wait_warp(&bar_kv_full[slot_of(uv)], par_of(uv), abort_p)) { ok = false; break; }
-        tr.mark(10);
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-          if (j < ntile[q]) {
-            const int sb = (NS == 2) ? (j & 1) : 0;
-            const uint32_t par = (NS == 2) ? ((j >> 1) & 1) : (j & 1);
-            static_for<0, kPvParts>([&](auto h_) {
-              constexpr int h = decltype(h_)::value;
-              if (ok) {
-                if (!mbar_wait_warp(&bar_p_ready[(q * NS + sb) * kPvParts + h], par, abort_p)) {
-                  ok = false;
-                } else {
-                  if (h == 0) tr.mark(11 + 2 * q);
-                  tc_fence_after_sync();
-                  issue_pv<DP, BN, 2 * h, 2 * h + 2>(o_tm(q), s_tm(q, sb), v_lo(uv), idesc_pv,
-                                                     (h > 0) || (j > 0) || (p.first == 0), el);
-                }
-              }
-            });
-            if (!ok) break;
-            if (NS == 2 || j + 1 == ntile[q]) mma_commit_e(&bar_pv_done[q], el);
-            if (NS == 1 && j + 1 < ntile[q]) {
+            for (int pn = 0; pn < Cfg::kPanels; ++pn)
+              tma_load_4d(s_q + q * Cfg::kQBytes + pn * (128 * 128), &tm_q, &bar_q_full, pn * 64, h, m0[q], b);
+          }
+        }
+        bool ok = true;
+        for (int j = 0; j < nmax && ok; ++j) {
+#pragma unroll
+          for (int which = 0; which < 2; ++which) {
+            const int u = 2 * j + which;
+            const int slot = u % kSlots;
+            const int round = u / kSlots;
+            if (!mbar_wait(&bar_kv_empty[slot], (round & 1) ^ 1, abort_p)) {
+              ok = false;
+              break;
+            }
+            tr.mark(40 + which);
+            mbar_expect_tx(&bar_kv_full[slot], Cfg::kKVBytes);
+#pragma unroll
+            for (int pn = 0; pn < Cfg::kPanels; ++pn)
+              tma_load_4d(s_kv + slot * Cfg::kKVBytes + pn * (BN * 128), which ? &tm_v : &tm_k, &bar_kv_full[slot],
+                          pn * 64, hkv, j * BN, b);
+          }
+        }
+      }
+      __syncwarp();
+    } else if (warp == 1) {
+      // =========================== MMA issuer ===========================
+      // The whole warp runs this loop converged; the elected lane issues.  A commit makes its mbarrier track every MMA
+      // issued before it, so the arrival on bar_s_full for tile j+1 also tells the softmax warps that O += P_j V_j has
+      // retired; bar_pv_done is only needed after the last tile.
+      {
+        const uint32_t el = elect_one();
+        constexpr uint32_t idesc_qk = make_idesc(128, BN, kBf16, false, false);
+        constexpr uint32_t idesc_pv = make_idesc(128, DP, kBf16, false, true);
+        auto slot_of = [&](int u) { return u % kSlots; };
+        auto par_of = [&](int u) { return static_cast<uint32_t>((u / kSlots) & 1); };
+        // descriptor low words of the operand tiles (K: K-major, V: MN-major, Q: K-major)
+        auto k_lo = [&](int u) { return desc_lo_kmajor(s_kv + slot_of(u) * Cfg::kKVBytes); };
+        auto v_lo = [&](int u) { return desc_lo_mnmajor(s_kv + slot_of(u) * Cfg::kKVBytes, BN * 128); };
+        uint32_t q_lo[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) q_lo[q] = desc_lo_kmajor(s_q + q * Cfg::kQBytes);
+        auto s_tm = [&](int q, int sb) { return tmem_base + Cfg::kTmS + (q * NS + sb) * BN; };
+        auto o_tm = [&](int q) { return tmem_base + Cfg::kTmO + q * DP; };
+        bool ok = nmax > 0;
+        if (ok) ok = mbar_wait_warp(&bar_q_full, 0, abort_p);
+        if (ok) ok = mbar_wait_warp(&bar_kv_full[slot_of(0)], par_of(0), abort_p);
+        if (ok) {
+          tc_fence_after_sync();
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) {
+            if (ntile[q] > 0) {
+              issue_qk<DP, BN>(s_tm(q, 0), q_lo[q], k_lo(0), idesc_qk, el);
+              mma_commit_e(&bar_s_full[q * NS + 0], el);
+            }
+          }
+          mma_commit_e(&bar_kv_empty[slot_of(0)], el);
+        }
+        for (int j = 0; j < nmax && ok; ++j) {
+          if (NS == 2) {
+            // Score buffer (j+1)&1 is free: P_{j-1} was consumed by the PV issued last iteration.
+            if (j + 1 < ntile[0]) {
               const int uk = 2 * (j + 1);
               if (!mbar_wait_warp(&bar_kv_full[slot_of(uk)], par_of(uk), abort_p)) { ok = false; break; }
               tc_fence_after_sync();
-              issue_qk<DP, BN>(s_tm(q, 0), q_lo[q], k_lo(uk), idesc_qk, el);
-              mma_commit_e(&bar_s_full[q * NS + 0], el);
+              issue_qk<DP, BN>(s_tm(0, (j + 1) & 1), q_lo[0], k_lo(uk), idesc_qk, el);
+              mma_commit_e(&bar_s_full[(j + 1) & 1], el);
+              mma_commit_e(&bar_kv_empty[slot_of(uk)], el);
             }
-            tr.mark(12 + 2 * q);
           }
+          const int uv = 2 * j + 1;
+          tr.mark(9);
+          if (!mbar_wait_warp(&bar_kv_full[slot_of(uv)], par_of(uv), abort_p)) { ok = false; break; }
+          tr.mark(10);
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) {
+            if (j < ntile[q]) {
+              const int sb = (NS == 2) ? (j & 1) : 0;
+              const uint32_t par = (NS == 2) ? ((j >> 1) & 1) : (j & 1);
+              static_for<0, kPvParts>([&](auto h_) {
+                constexpr int h = decltype(h_)::value;
+                if (ok) {
+                  if (!mbar_wait_warp(&bar_p_ready[(q * NS + sb) * kPvParts + h], par, abort_p)) {
+                    ok = false;
+                  } else {
+                    if (h == 0) tr.mark(11 + 2 * q);
+                    tc_fence_after_sync();
+                    issue_pv<DP, BN, 2 * h, 2 * h + 2>(o_tm(q), s_tm(q, sb), v_lo(uv), idesc_pv,
+                                                       (h > 0) || (j > 0) || (p.first == 0), el);
+                  }
+                }
+              });
+              if (!ok) break;
+              if (NS == 2 || j + 1 == ntile[q]) mma_commit_e(&bar_pv_done[q], el);
+              if (NS == 1 && j + 1 < ntile[q]) {
+                const int uk = 2 * (j + 1);
+                if (!mbar_wait_warp(&bar_kv_full[slot_of(uk)], par_of(uk), abort_p)) { ok = false; break; }
+                tc_fence_after_sync();
+                issue_qk<DP, BN>(s_tm(q, 0), q_lo[q], k_lo(uk), idesc_qk, el);
+                mma_commit_e(&bar_s_full[q * NS + 0], el);
+              }
+              tr.mark(12 + 2 * q);
+            }
+          }
+          if (!ok) break;
+          mma_commit_e(&bar_kv_empty[slot_of(uv)], el);
+          if (NS == 1 && j + 1 < nmax) mma_commit_e(&bar_kv_empty[slot_of(2 * (j + 1))], el);
         }
-        if (!ok) break;
-        mma_commit_e(&bar_kv_empty[slot_of(uv)], el);
-        if (NS == 1 && j + 1 < nmax) mma_commit_e(&bar_kv_empty[slot_of(2 * (j + 1))], el);
       }
+      __syncwarp();
     }
-    __syncwarp();
-  } else if (warp >= 4) {
+  } else {
     // =========================== softmax warpgroups ===========================
+    if constexpr (NQ == 2) setmaxnreg_inc<Cfg::kSoftmaxRegs>();
     const int q = (warp - 4) >> 2;
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const int n = ntile[q];
-    const int row_g = m0[q] + row;  // local query position
+    // selected, not indexed: an array indexed at run time would live in local memory for the issuer as well
+    const int n = (NQ == 2 && q == 1) ? ntile[NQ - 1] : ntile[0];
+    const int m0_q = (NQ == 2 && q == 1) ? m0[NQ - 1] : m0[0];
+    const int row_g = m0_q + row;  // local query position
     const uint32_t o_addr = tmem_base + lane_addr + Cfg::kTmO + q * DP;
     const int qt = tq0 + qs * NQ + q;
-    const bool last_here = (m0[q] < p.q_split) ? (p.last_lo != 0) : (p.last != 0);
+    const bool last_here = (m0_q < p.q_split) ? (p.last_lo != 0) : (p.last != 0);
     const size_t bh = static_cast<size_t>(b) * p.Hq + h;
     float* acc_tile = p.acc + ((bh * p.nQt + qt) * (DP / 4)) * 512;  // [DP/4][128][4]
     const size_t ml_idx = bh * p.Spad + row_g;
@@ -346,7 +359,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
         tc_fence_after_sync();
         const uint32_t s_addr = tmem_base + lane_addr + Cfg::kTmS + (q * NS + sb) * BN;
         const int n0 = j * BN;
-        const bool masked = (p.causal && (n0 + BN - 1 > m0[q])) || (n0 + BN > p.kv_len);
+        const bool masked = (p.causal && (n0 + BN - 1 > m0_q)) || (n0 + BN > p.kv_len);
 
         // The whole score row (BN fp32 values) goes to registers in one batch of loads.
         constexpr int NCH = BN / 32;
@@ -371,10 +384,11 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
           mxp[c][0] = __uint_as_float(r[c][0]);
           mxp[c][1] = __uint_as_float(r[c][1]);
 #pragma unroll
-          for (int i = 2; i < 32; i += 2) {
-            mxp[c][0] = fmaxf(mxp[c][0], __uint_as_float(r[c][i]));
-            mxp[c][1] = fmaxf(mxp[c][1], __uint_as_float(r[c][i + 1]));
+          for (int i = 2; i < 30; i += 4) {
+            mxp[c][0] = max3(mxp[c][0], __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
+            mxp[c][1] = max3(mxp[c][1], __uint_as_float(r[c][i + 2]), __uint_as_float(r[c][i + 3]));
           }
+          mxp[c][0] = max3(mxp[c][0], __uint_as_float(r[c][30]), __uint_as_float(r[c][31]));
         }
         float mx = fmaxf(mxp[0][0], mxp[0][1]);
 #pragma unroll
@@ -549,6 +563,14 @@ static int launch_fwd(const void* q, const void* k, const void* v, const FwdPara
   if (!attr_done[traced][dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
     if (e != cudaSuccess) { cudaGetLastError(); return RFA_ERR_CUDA; }
+    if (NQ == 2) {
+      // A raise that the launch's pool (threads x registers per thread) cannot satisfy would wait forever: a build whose
+      // register count does not cover the allowances is refused.
+      cudaFuncAttributes fa;
+      e = cudaFuncGetAttributes(&fa, kern);
+      if (e != cudaSuccess) { cudaGetLastError(); return RFA_ERR_CUDA; }
+      if (fa.numRegs * Cfg::kThreads < Cfg::kPoolRegs) return RFA_ERR_UNSUPPORTED;
+    }
     attr_done[traced][dev] = true;
   }
   const int nQs = (prm.nQt - prm.q_begin / 128 + NQ - 1) / NQ;

@@ -539,6 +539,13 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// Largest of three (one instruction on sm_100; the non-NaN operand wins, as with fmaxf).
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+
 // Packed pairs of fp32 (Blackwell add/fma .f32x2: one issue slot for two lanes of arithmetic).
 __device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
   uint64_t r;
