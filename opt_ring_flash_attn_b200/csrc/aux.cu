@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "common.h"
+#include "tc05.cuh"
 
 namespace rfa {
 
@@ -92,6 +93,8 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const T* __restrict__ 
                                                          const float* __restrict__ lse, float* __restrict__ delta,
                                                          float* __restrict__ lse2, int B, int Sq, int Spad, int Hq,
                                                          int D, const ClearList clear) {
+  pdl_wait();
+  pdl_trigger();
   {
     const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
 #pragma unroll
@@ -182,6 +185,7 @@ __global__ void __launch_bounds__(256) dq_finalize_kernel(const float* __restric
                                                          int Sq, int Hq, int D, int DP, int nQt, int dq_blocks,
                                                          const float* __restrict__ dkdv, T* __restrict__ dk,
                                                          T* __restrict__ dv, size_t n8) {
+  pdl_wait();
   if (static_cast<int>(blockIdx.x) >= dq_blocks) {
     const size_t i0 = static_cast<size_t>(blockIdx.x - dq_blocks) * kCastVec + threadIdx.x;
 #pragma unroll
@@ -330,13 +334,12 @@ int launch_bwd_prepare(const void* out, const void* dout, const float* lse, floa
   if (blocks > 148ll * 16) blocks = 148ll * 16;
   if (blocks < 1) blocks = 1;
   if (dtype == RFA_DTYPE_BF16)
-    bwd_prepare_kernel<__nv_bfloat16><<<static_cast<unsigned>(blocks), threads, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), lse, delta, lse2, B, Sq, Spad,
-        Hq, D, clear);
-  else
-    bwd_prepare_kernel<__half><<<static_cast<unsigned>(blocks), threads, 0, s>>>(
-        static_cast<const __half*>(out), static_cast<const __half*>(dout), lse, delta, lse2, B, Sq, Spad, Hq, D, clear);
-  return cuda_status(cudaGetLastError());
+    return launch_chained(bwd_prepare_kernel<__nv_bfloat16>, static_cast<unsigned>(blocks), threads, 0, s,
+                          static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), lse, delta,
+                          lse2, B, Sq, Spad, Hq, D, clear);
+  return launch_chained(bwd_prepare_kernel<__half>, static_cast<unsigned>(blocks), threads, 0, s,
+                        static_cast<const __half*>(out), static_cast<const __half*>(dout), lse, delta, lse2, B, Sq, Spad,
+                        Hq, D, clear);
 }
 
 int launch_bwd_finish(const float* dq_acc, void* dq, const float* dkdv, void* dk, void* dv, int B, int Sq, int Skv, int Hq,
@@ -347,14 +350,11 @@ int launch_bwd_finish(const float* dq_acc, void* dq, const float* dkdv, void* dk
   const size_t n8 = dkdv ? static_cast<size_t>(B) * Skv * Hkv * D / 8 : 0;
   const unsigned grid = dq_blocks + static_cast<unsigned>((2 * n8 + kCastVec - 1) / kCastVec);
   if (dtype == RFA_DTYPE_BF16)
-    dq_finalize_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(
-        dq_acc, static_cast<__nv_bfloat16*>(dq), B, Sq, Hq, D, dp, nQt, static_cast<int>(dq_blocks), dkdv,
-        static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), n8);
-  else
-    dq_finalize_kernel<__half><<<grid, 256, 0, s>>>(dq_acc, static_cast<__half*>(dq), B, Sq, Hq, D, dp, nQt,
-                                                    static_cast<int>(dq_blocks), dkdv, static_cast<__half*>(dk),
-                                                    static_cast<__half*>(dv), n8);
-  return cuda_status(cudaGetLastError());
+    return launch_chained(dq_finalize_kernel<__nv_bfloat16>, grid, 256, 0, s, dq_acc, static_cast<__nv_bfloat16*>(dq), B,
+                          Sq, Hq, D, dp, nQt, static_cast<int>(dq_blocks), dkdv, static_cast<__nv_bfloat16*>(dk),
+                          static_cast<__nv_bfloat16*>(dv), n8);
+  return launch_chained(dq_finalize_kernel<__half>, grid, 256, 0, s, dq_acc, static_cast<__half*>(dq), B, Sq, Hq, D, dp,
+                        nQt, static_cast<int>(dq_blocks), dkdv, static_cast<__half*>(dk), static_cast<__half*>(dv), n8);
 }
 
 }  // namespace rfa

@@ -131,9 +131,7 @@ __global__ void __launch_bounds__(640, 1)
   __shared__ uint64_t bar_q_full[NSQ], bar_q_empty[NSQ], bar_do_full[NSO], bar_do_empty[NSO];
   __shared__ uint64_t bar_s_full, bar_p_ready, bar_dp_full, bar_ds_ready, bar_dq_full, bar_dq_drained, bar_final;
   __shared__ uint32_t tmem_holder;
-  __shared__ int abort_flag;
-
-  if (*reinterpret_cast<volatile int*>(p.status) != 0) return;
+  __shared__ int abort_flag, skip_flag;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -212,10 +210,16 @@ __global__ void __launch_bounds__(640, 1)
     tmem_alloc(&tmem_holder, 512);
     tmem_relinquish();
   }
+  pdl_wait();  // nothing above touches global memory
+  if (tid == 0) skip_flag = *reinterpret_cast<volatile int*>(p.status);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_holder;
+  if (skip_flag != 0) {  // an earlier kernel gave up
+    if (warp == 0) tmem_dealloc(tmem_base, 512);
+    return;
+  }
   volatile int* abort_p = &abort_flag;
   const bool run = (abort_flag == 0) && (T_total > 0);
 
@@ -822,8 +826,7 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
   }
   const long long base_units = static_cast<long long>(ceil_div(prm.kv_len, 128)) * prm.Hkv * prm.B * Cfg::kHalves;
   const unsigned grid = static_cast<unsigned>(base_units * prm.nsplit);
-  kern<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv, tdo, prm);
-  return cuda_status(cudaGetLastError());
+  return launch_chained(kern, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, tq, tk, tv, tdo, prm);
 }
 
 template <typename T>

@@ -59,6 +59,29 @@ int launch_bwd_finish(const float* dq_acc, void* dq, const float* dkdv, void* dk
                       int Hkv, int D, int dtype, cudaStream_t stream);
 
 // Translates a CUDA runtime error into an ABI error code (and clears it).
-inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? RFA_OK : RFA_ERR_CUDA; }
+inline int cuda_status(cudaError_t e) {
+  if (e == cudaSuccess) return RFA_OK;
+  cudaGetLastError();
+  return RFA_ERR_CUDA;
+}
+
+// Launches a kernel whose blocks may start while the previous kernel of the stream drains.  Such a kernel calls
+// pdl_wait() before it touches global memory, so that what it reads is complete and what it overwrites is no longer
+// read; what comes before (barriers, tensor memory, descriptors) overlaps the predecessor's tail.
+template <typename... P, typename... A>
+inline int launch_chained(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream,
+                          const A&... args) {
+  cudaLaunchAttribute attr[1] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cuda_status(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+}
 
 }  // namespace rfa

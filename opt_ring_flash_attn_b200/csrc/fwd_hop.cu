@@ -106,9 +106,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
   __shared__ uint64_t bar_p_ready[NQ * NS * kPvParts];  // [score buffer][part of the keys]
   __shared__ uint64_t bar_pv_done[NQ];
   __shared__ uint32_t tmem_holder;
-  __shared__ int abort_flag;
-
-  if (*reinterpret_cast<volatile int*>(p.status) != 0) return;  // an earlier kernel gave up
+  __shared__ int abort_flag, skip_flag;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -162,10 +160,16 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
     tmem_alloc(&tmem_holder, 512);
     tmem_relinquish();
   }
+  pdl_wait();  // nothing above touches global memory
+  if (tid == 0) skip_flag = *reinterpret_cast<volatile int*>(p.status);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_holder;
+  if (skip_flag != 0) {  // an earlier kernel gave up
+    if (warp == 0) tmem_dealloc(tmem_base, 512);
+    return;
+  }
   volatile int* abort_p = &abort_flag;
   Tracer<kTrace> tr;
   {
@@ -575,8 +579,7 @@ static int launch_fwd(const void* q, const void* k, const void* v, const FwdPara
   }
   const int nQs = (prm.nQt - prm.q_begin / 128 + NQ - 1) / NQ;
   const unsigned grid = static_cast<unsigned>(nQs) * prm.Hq * prm.B;
-  kern<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv, prm);
-  return cuda_status(cudaGetLastError());
+  return launch_chained(kern, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, tq, tk, tv, prm);
 }
 
 template <typename T>

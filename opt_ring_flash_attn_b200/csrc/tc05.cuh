@@ -48,6 +48,11 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
   return t;
 }
 
+// Programmatic dependent launch: wait until the previous kernel of the stream is complete and its writes are visible /
+// let the next kernel's blocks start (they wait in turn).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------
 // mbarrier
 // ----------------------------------------------------------------------------
