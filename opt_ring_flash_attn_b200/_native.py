@@ -119,7 +119,9 @@ def _stream(stream: Optional[torch.cuda.Stream], ref: Optional[torch.Tensor] = N
     """Raw stream handle: the given stream, else the current stream of ``ref``'s device."""
     if stream is not None:
         return stream.cuda_stream
-    return torch.cuda.current_stream(ref.device if ref is not None else None).cuda_stream
+    # the handle alone: a Stream object costs 2 us to make, twice per pass
+    device = ref.device.index if ref is not None else None
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device is None else device)
 
 
 _NO_GUARD = contextlib.nullcontext()

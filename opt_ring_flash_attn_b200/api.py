@@ -96,7 +96,7 @@ class _RingFlashAttnFunc(torch.autograd.Function):
             assert causal, "zigzag mode requires causal=True"
         _validate(q, k, v, softmax_scale)
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        ctx.balanced = bool(causal and not zigzag and _balanced_now() and schedule.can_balance(group, q.shape[1]))
+        ctx.balanced = bool(causal and not zigzag and schedule.can_balance(group, q.shape[1]) and _balanced_now())
         if ctx.balanced:
             out, lse, saved = schedule.balanced_forward(group, q, k, v, softmax_scale)
             ctx.save_for_backward(*saved)  # the zigzag-arranged q, k, v, out, lse
@@ -112,11 +112,15 @@ class _RingFlashAttnFunc(torch.autograd.Function):
         ctx.group = group
         ctx.deterministic = _deterministic_now()
         ctx.mark_non_differentiable(lse)
+        # the gradient of lse is never used: without this autograd fills a tensor with zeros for it on every backward
+        ctx.set_materialize_grads(False)
         return out, lse
 
     @staticmethod
     def backward(ctx, dout, _dlse=None):
         q, k, v, out, lse = ctx.saved_tensors
+        if dout is None:
+            dout = torch.zeros_like(out)
         if ctx.balanced:
             dq, dk, dv = schedule.balanced_backward(ctx.group, dout, (q, k, v, out, lse), ctx.softmax_scale,
                                                     deterministic=ctx.deterministic)

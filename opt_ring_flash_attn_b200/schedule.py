@@ -130,22 +130,53 @@ def _world(group) -> Tuple[int, int]:
     return 1, 0
 
 
+def _local_forward(kn, group, q, k, v, softmax_scale: float, causal: bool):
+    """The forward pass of a shard without a ring: one hop, nothing to carry."""
+    ws = workspace.forward_workspace(q, k, 1, owner=_ws_owner(group))
+    workspace.raise_if_failed(ws, "ring_flash_attn forward")
+    B, S, Hq, _ = q.shape
+    out = torch.empty_like(q)
+    lse = torch.empty((B, Hq, _native.padded_seq(S)), dtype=torch.float32, device=q.device)
+    kn.fwd_hop(q, k, v, None, None, None, out, lse, softmax_scale, True, True, causal, ws.status)
+    workspace.publish_status(ws, "ring_flash_attn forward")
+    return out, lse
+
+
+def _local_backward(kn, group, dout, q, k, v, out, lse, softmax_scale: float, causal: bool, deterministic: bool):
+    """The backward pass of a shard without a ring: nothing happens between the kernels, one call enqueues them all."""
+    ws = workspace.backward_workspace(q, k, 1, owner=_ws_owner(group))
+    workspace.raise_if_failed(ws, "ring_flash_attn backward")
+    dout = dout.contiguous()
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    order = ws.dq_order if deterministic else None
+    if hasattr(kn, "bwd_local"):
+        kn.bwd_local(q, k, v, out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.dkdv[0], dq, dk, dv, softmax_scale,
+                     causal, ws.status, dq_order=order)
+    else:  # a kernel backend that only has the parts
+        buf = ws.dkdv[0]
+        kn.bwd_prepare(out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.status)
+        kn.bwd_hop(q, k, v, dout, ws.lse2, ws.delta, ws.dq_acc, None, buf, softmax_scale, False, causal, ws.status,
+                   dq_order=order)
+        kn.dq_finalize(ws.dq_acc, dq)
+        kn.cast_from_f32(buf[0], dk)
+        kn.cast_from_f32(buf[1], dv)
+    workspace.publish_status(ws, "ring_flash_attn backward")
+    return dq, dk, dv
+
+
 def ring_forward(group, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, softmax_scale: float, causal: bool,
                  kernels=None) -> Tuple[torch.Tensor, torch.Tensor]:
     """Returns ``(out [B,S,Hq,D] in q's dtype, lse_padded [B,Hq,Spad] fp32)``; both are fresh tensors."""
     kn = kernels if kernels is not None else _native
     W, rank = _world(group)
+    if W == 1:
+        return _local_forward(kn, group, q, k, v, softmax_scale, causal)
     B, S, Hq, D = q.shape
     _agree_on_shapes(group, q, k, W)
     ws = workspace.forward_workspace(q, k, W, owner=_ws_owner(group), ring=_ring_factory(group, q.device))
     workspace.raise_if_failed(ws, "ring_flash_attn forward")
     out = torch.empty_like(q)
     lse = torch.empty(B, Hq, _native.padded_seq(S), dtype=torch.float32, device=q.device)
-
-    if W == 1:
-        kn.fwd_hop(q, k, v, None, None, None, out, lse, softmax_scale, True, True, causal, ws.status)
-        workspace.publish_status(ws, "ring_flash_attn forward")
-        return out, lse
 
     comm = ws.comms["fwd_kv"]
     kn.pack_kv(k, v, ws.kv_send)
@@ -202,6 +233,8 @@ def ring_backward(group, dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v
     optimized_ring_flash_attn.py:730-735) at some cost in speed."""
     kn = kernels if kernels is not None else _native
     W, rank = _world(group)
+    if W == 1:
+        return _local_backward(kn, group, dout, q, k, v, out, lse, softmax_scale, causal, deterministic)
     ws = workspace.backward_workspace(q, k, W, backward_comm_dtype(q.dtype), owner=_ws_owner(group),
                                       ring=_ring_factory(group, q.device))
     workspace.raise_if_failed(ws, "ring_flash_attn backward")
@@ -211,24 +244,7 @@ def ring_backward(group, dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v
     dq = torch.empty_like(q)
     dk = torch.empty_like(k)
     dv = torch.empty_like(v)
-    if W == 1 and hasattr(kn, "bwd_local"):
-        # nothing happens between the kernels: one call enqueues them all
-        kn.bwd_local(q, k, v, out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.dkdv[0], dq, dk, dv, softmax_scale,
-                     causal, ws.status, **order)
-        workspace.publish_status(ws, "ring_flash_attn backward")
-        return dq, dk, dv
-
     kn.bwd_prepare(out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.status)
-    if W == 1:
-        buf = ws.dkdv[0]
-        kn.bwd_hop(q, k, v, dout, ws.lse2, ws.delta, ws.dq_acc, None, buf, softmax_scale, False, causal, ws.status,
-                   **order)
-        kn.dq_finalize(ws.dq_acc, dq)
-        kn.cast_from_f32(buf[0], dk)
-        kn.cast_from_f32(buf[1], dv)
-        workspace.publish_status(ws, "ring_flash_attn backward")
-        return dq, dk, dv
-
     kv_comm, dkv_comm = ws.comms["bwd_kv"], ws.comms["bwd_dkdv"]
     kn.pack_kv(k, v, ws.kv_send)
     cur = ws.kv_send
@@ -282,16 +298,14 @@ def zigzag_forward(group, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, sof
     """
     kn = kernels if kernels is not None else _native
     W, rank = _world(group)
+    if W == 1:
+        return _local_forward(kn, group, q, k, v, softmax_scale, True)
     B, S, Hq, D = q.shape
     _agree_on_shapes(group, q, k, W)
     ws = workspace.forward_workspace(q, k, W, owner=_ws_owner(group), ring=_ring_factory(group, q.device))
     workspace.raise_if_failed(ws, "ring_flash_attn forward")
     out = torch.empty_like(q)
     lse = torch.empty(B, Hq, _native.padded_seq(S), dtype=torch.float32, device=q.device)
-    if W == 1:
-        kn.fwd_hop(q, k, v, None, None, None, out, lse, softmax_scale, True, True, True, ws.status)
-        workspace.publish_status(ws, "ring_flash_attn forward")
-        return out, lse
     half = _zigzag_half(S)
     comm = ws.comms["fwd_kv"]
     kn.pack_kv(k, v, ws.kv_send)

@@ -70,7 +70,7 @@ _bwd_cache: Dict[Any, Tuple[Tuple, BackwardWorkspace]] = {}
 
 
 def _key(q: torch.Tensor, k: torch.Tensor, world_size: int, extra=None) -> Tuple:
-    return (tuple(q.shape), tuple(k.shape), q.dtype, str(q.device), world_size, extra)
+    return (q.shape, k.shape, q.dtype, q.device, world_size, extra)
 
 
 def _new_status(dev: torch.device):
