@@ -480,6 +480,9 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
       }
 
       // ---- epilogue: wait for the last PV, then spill state or write the result ----
+      // With two score buffers the last scores only prove that O += P_{n-3} V_{n-3} has retired: a wait for the parity of
+      // the last product alone would also be satisfied by the phase before the one of tile n-2.
+      if (NS == 2 && ok && n > 1) ok = mbar_wait_warp(&bar_pv_done[q], (n - 2) & 1, abort_p);
       if (ok) ok = mbar_wait_warp(&bar_pv_done[q], (NS == 2) ? ((n - 1) & 1) : 0, abort_p);
       if (ok) {
         tc_fence_after_sync();
