@@ -14,8 +14,12 @@
 //               reads S from tensor memory, exp2-domain online softmax with lazy
 //               rescaling of O, writes P (16-bit) back over S.
 // Tensor memory: [0, NQ*DP) O accumulators, then NQ*NS score buffers of BN columns.
-// Two variants: NQ=2 Q tiles with one score buffer each (D <= 128), and NQ=1 with
-// two alternating score buffers and BN=64 (D = 256).
+// Two variants: NQ=2 Q tiles with one score buffer each (D <= 128), and NQ=1 with two alternating score buffers (D = 256),
+// where a K/V tile is loaded in two pieces of 128 head-dim columns: five pieces of 32 KB fit beside Q, and they arrive
+// and are released in the order in which the products use them (K0, K1, V0, K2, V1, ...).  Tiles of 64 keys, four whole
+// slots, needed no pieces, but S = Q K^T with 64 columns reads 6 KB of operands per 32 tensor cycles, more than shared
+// memory delivers, and Q twice as often: full block of B 2,
+// S 4096, 16 heads 629 us, diagonal 333; with pieces 517 and 291.
 #include "common.h"
 #include "tc05.cuh"
 
@@ -50,8 +54,9 @@ struct FwdCfg {
   static constexpr int kBM = 128;
   static constexpr int kPanels = DP / 64;
   static constexpr int kQBytes = kBM * DP * 2;
-  static constexpr int kKVBytes = BN * DP * 2;
-  static constexpr int kSlots = (DP == 64) ? 8 : 4;
+  static constexpr int kPieces = (NS == 2) ? DP / 128 : 1;  // a K/V tile arrives in as many slots
+  static constexpr int kKVBytes = BN * DP * 2 / kPieces;
+  static constexpr int kSlots = (DP == 64) ? 8 : (NS == 2) ? 5 : 4;
   static constexpr int kSmemTiles = NQ * kQBytes + kSlots * kKVBytes;
   static constexpr int kSmemBytes = kSmemTiles + 1024;  // slack for 1024-byte alignment
   static constexpr int kThreads = 128 + NQ * 128;
@@ -67,12 +72,12 @@ struct FwdCfg {
 // S[128 x BN] = Q[128 x DP] * K[BN x DP]^T, both operands K-major.
 template <int DP, int BN>
 __device__ __forceinline__ void issue_qk(uint32_t s_tmem, uint32_t q_smem, uint32_t k_smem, uint32_t idesc,
-                                         uint32_t el) {
+                                         uint32_t el, bool accumulate = false) {
   // q_smem / k_smem are descriptor low words of the tile bases; offsets are in 16-byte units
   static_for<0, DP / 16>([&](auto ks_) {
     constexpr int ks = decltype(ks_)::value;
     mma_ss_off_e<(((ks / 4) * (128 * 128) + (ks % 4) * 32) / 16), (((ks / 4) * (BN * 128) + (ks % 4) * 32) / 16)>(
-        s_tmem, q_smem, k_smem, idesc, ks > 0 ? 1u : 0u, el);
+        s_tmem, q_smem, k_smem, idesc, (accumulate || ks > 0) ? 1u : 0u, el);
   });
 }
 
@@ -87,6 +92,19 @@ __device__ __forceinline__ void issue_pv(uint32_t o_tmem, uint32_t p_tmem, uint3
     mma_ts_off_e<(ks * 8), (ks * 128)>(o_tmem, p_tmem, v_smem, idesc, (accumulate || ks > KS0) ? 1u : 0u, el);
   });
 }
+
+// Position in the ring of K/V slots, advanced one slot at a time (for a count that is no power of two).
+template <int kSlots>
+struct SlotWalk {
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++slot == kSlots) {
+      slot = 0;
+      phase ^= 1;
+    }
+  }
+};
 
 template <int DP, int BN, int NQ, int NS, typename T, bool kTrace>
 __global__ void __launch_bounds__(128 + NQ * 128, 1)
@@ -203,7 +221,25 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
           }
         }
         bool ok = true;
-        for (int j = 0; j < nmax && ok; ++j) {
+        if constexpr (NS == 2) {
+          SlotWalk<kSlots> w;
+          auto load = [&](int which, int j) {
+#pragma unroll
+            for (int pc = 0; pc < Cfg::kPieces; ++pc, w.next()) {
+              if (!mbar_wait(&bar_kv_empty[w.slot], w.phase ^ 1, abort_p)) return false;
+              tr.mark(40 + which);
+              mbar_expect_tx(&bar_kv_full[w.slot], Cfg::kKVBytes);
+#pragma unroll
+              for (int pn = 0; pn < 2; ++pn)
+                tma_load_4d(s_kv + w.slot * Cfg::kKVBytes + pn * (BN * 128), which ? &tm_v : &tm_k, &bar_kv_full[w.slot],
+                            (2 * pc + pn) * 64, hkv, j * BN, b);
+            }
+            return true;
+          };
+          ok = nmax > 0 && load(0, 0);
+          for (int j = 0; j < nmax && ok; ++j) ok = (j + 1 == nmax || load(0, j + 1)) && load(1, j);
+        }
+        for (int j = 0; NS == 1 && j < nmax && ok; ++j) {
 #pragma unroll
           for (int which = 0; which < 2; ++which) {
             const int u = 2 * j + which;
@@ -228,7 +264,61 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
       // The whole warp runs this loop converged; the elected lane issues.  A commit makes its mbarrier track every MMA
       // issued before it, so the arrival on bar_s_full for tile j+1 also tells the softmax warps that O += P_j V_j has
       // retired; bar_pv_done is only needed after the last tile.
-      {
+      if constexpr (NS == 2) {
+        const uint32_t el = elect_one();
+        constexpr uint32_t idesc_qk = make_idesc(128, BN, kBf16, false, false);
+        constexpr uint32_t idesc_pv = make_idesc(128, 128, kBf16, false, true);
+        const uint32_t q_lo = desc_lo_kmajor(s_q);
+        SlotWalk<kSlots> w;
+        auto s_tm = [&](int j) { return tmem_base + Cfg::kTmS + (j & 1) * BN; };
+        auto qk = [&](int j) {
+          bool got = true;
+          static_for<0, Cfg::kPieces>([&](auto pc_) {
+            constexpr int pc = decltype(pc_)::value;
+            if (!got) return;
+            got = mbar_wait_warp(&bar_kv_full[w.slot], w.phase, abort_p);
+            if (!got) return;
+            tc_fence_after_sync();
+            issue_qk<128, BN>(s_tm(j), q_lo + pc * (2 * 128 * 128 / 16), desc_lo_kmajor(s_kv + w.slot * Cfg::kKVBytes),
+                              idesc_qk, el, pc > 0);
+            mma_commit_e(&bar_kv_empty[w.slot], el);
+            w.next();
+          });
+          if (got) mma_commit_e(&bar_s_full[j & 1], el);
+          return got;
+        };
+        bool ok = nmax > 0 && mbar_wait_warp(&bar_q_full, 0, abort_p) && qk(0);
+        for (int j = 0; j < nmax && ok; ++j) {
+          // Score buffer (j+1)&1 is free: P_{j-1} was consumed by the PV issued last iteration.
+          if (j + 1 < nmax && !qk(j + 1)) break;
+          tr.mark(9);
+          uint32_t v_lo[Cfg::kPieces];
+          int v_slot[Cfg::kPieces];
+#pragma unroll
+          for (int pc = 0; pc < Cfg::kPieces; ++pc, w.next()) {
+            v_slot[pc] = w.slot;
+            v_lo[pc] = desc_lo_mnmajor(s_kv + w.slot * Cfg::kKVBytes, BN * 128);
+            ok = ok && mbar_wait_warp(&bar_kv_full[w.slot], w.phase, abort_p);
+          }
+          tr.mark(10);
+          static_for<0, kPvParts>([&](auto h_) {
+            constexpr int h = decltype(h_)::value;
+            ok = ok && mbar_wait_warp(&bar_p_ready[(j & 1) * kPvParts + h], (j >> 1) & 1, abort_p);
+            if (!ok) return;
+            if (h == 0) tr.mark(11);
+            tc_fence_after_sync();
+#pragma unroll
+            for (int pc = 0; pc < Cfg::kPieces; ++pc)
+              issue_pv<128, BN, 2 * h, 2 * h + 2>(tmem_base + Cfg::kTmO + pc * 128, s_tm(j), v_lo[pc], idesc_pv,
+                                                  (h > 0) || (j > 0) || (p.first == 0), el);
+          });
+          if (!ok) break;
+          mma_commit_e(&bar_pv_done[0], el);
+#pragma unroll
+          for (int pc = 0; pc < Cfg::kPieces; ++pc) mma_commit_e(&bar_kv_empty[v_slot[pc]], el);
+          tr.mark(12);
+        }
+      } else {
         const uint32_t el = elect_one();
         constexpr uint32_t idesc_qk = make_idesc(128, BN, kBf16, false, false);
         constexpr uint32_t idesc_pv = make_idesc(128, DP, kBf16, false, true);
@@ -240,7 +330,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
         uint32_t q_lo[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q) q_lo[q] = desc_lo_kmajor(s_q + q * Cfg::kQBytes);
-        auto s_tm = [&](int q, int sb) { return tmem_base + Cfg::kTmS + (q * NS + sb) * BN; };
+        auto s_tm = [&](int q) { return tmem_base + Cfg::kTmS + q * BN; };
         auto o_tm = [&](int q) { return tmem_base + Cfg::kTmO + q * DP; };
         bool ok = nmax > 0;
         if (ok) ok = mbar_wait_warp(&bar_q_full, 0, abort_p);
@@ -250,24 +340,13 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
 #pragma unroll
           for (int q = 0; q < NQ; ++q) {
             if (ntile[q] > 0) {
-              issue_qk<DP, BN>(s_tm(q, 0), q_lo[q], k_lo(0), idesc_qk, el);
-              mma_commit_e(&bar_s_full[q * NS + 0], el);
+              issue_qk<DP, BN>(s_tm(q), q_lo[q], k_lo(0), idesc_qk, el);
+              mma_commit_e(&bar_s_full[q], el);
             }
           }
           mma_commit_e(&bar_kv_empty[slot_of(0)], el);
         }
         for (int j = 0; j < nmax && ok; ++j) {
-          if (NS == 2) {
-            // Score buffer (j+1)&1 is free: P_{j-1} was consumed by the PV issued last iteration.
-            if (j + 1 < ntile[0]) {
-              const int uk = 2 * (j + 1);
-              if (!mbar_wait_warp(&bar_kv_full[slot_of(uk)], par_of(uk), abort_p)) { ok = false; break; }
-              tc_fence_after_sync();
-              issue_qk<DP, BN>(s_tm(0, (j + 1) & 1), q_lo[0], k_lo(uk), idesc_qk, el);
-              mma_commit_e(&bar_s_full[(j + 1) & 1], el);
-              mma_commit_e(&bar_kv_empty[slot_of(uk)], el);
-            }
-          }
           const int uv = 2 * j + 1;
           tr.mark(9);
           if (!mbar_wait_warp(&bar_kv_full[slot_of(uv)], par_of(uv), abort_p)) { ok = false; break; }
@@ -275,36 +354,35 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
 #pragma unroll
           for (int q = 0; q < NQ; ++q) {
             if (j < ntile[q]) {
-              const int sb = (NS == 2) ? (j & 1) : 0;
-              const uint32_t par = (NS == 2) ? ((j >> 1) & 1) : (j & 1);
+              const uint32_t par = j & 1;
               static_for<0, kPvParts>([&](auto h_) {
                 constexpr int h = decltype(h_)::value;
                 if (ok) {
-                  if (!mbar_wait_warp(&bar_p_ready[(q * NS + sb) * kPvParts + h], par, abort_p)) {
+                  if (!mbar_wait_warp(&bar_p_ready[q * kPvParts + h], par, abort_p)) {
                     ok = false;
                   } else {
                     if (h == 0) tr.mark(11 + 2 * q);
                     tc_fence_after_sync();
-                    issue_pv<DP, BN, 2 * h, 2 * h + 2>(o_tm(q), s_tm(q, sb), v_lo(uv), idesc_pv,
+                    issue_pv<DP, BN, 2 * h, 2 * h + 2>(o_tm(q), s_tm(q), v_lo(uv), idesc_pv,
                                                        (h > 0) || (j > 0) || (p.first == 0), el);
                   }
                 }
               });
               if (!ok) break;
-              if (NS == 2 || j + 1 == ntile[q]) mma_commit_e(&bar_pv_done[q], el);
-              if (NS == 1 && j + 1 < ntile[q]) {
+              if (j + 1 == ntile[q]) mma_commit_e(&bar_pv_done[q], el);
+              if (j + 1 < ntile[q]) {
                 const int uk = 2 * (j + 1);
                 if (!mbar_wait_warp(&bar_kv_full[slot_of(uk)], par_of(uk), abort_p)) { ok = false; break; }
                 tc_fence_after_sync();
-                issue_qk<DP, BN>(s_tm(q, 0), q_lo[q], k_lo(uk), idesc_qk, el);
-                mma_commit_e(&bar_s_full[q * NS + 0], el);
+                issue_qk<DP, BN>(s_tm(q), q_lo[q], k_lo(uk), idesc_qk, el);
+                mma_commit_e(&bar_s_full[q], el);
               }
               tr.mark(12 + 2 * q);
             }
           }
           if (!ok) break;
           mma_commit_e(&bar_kv_empty[slot_of(uv)], el);
-          if (NS == 1 && j + 1 < nmax) mma_commit_e(&bar_kv_empty[slot_of(2 * (j + 1))], el);
+          if (j + 1 < nmax) mma_commit_e(&bar_kv_empty[slot_of(2 * (j + 1))], el);
         }
       }
       __syncwarp();
@@ -591,7 +669,7 @@ static int dispatch_fwd(int dp, const void* q, const void* k, const void* v, con
   switch (dp) {
     case 64: return launch_fwd<64, 128, 2, 1, T>(q, k, v, prm, dtype, stream);
     case 128: return launch_fwd<128, 128, 2, 1, T>(q, k, v, prm, dtype, stream);
-    case 256: return launch_fwd<256, 64, 1, 2, T>(q, k, v, prm, dtype, stream);
+    case 256: return launch_fwd<256, 128, 1, 2, T>(q, k, v, prm, dtype, stream);
     default: return RFA_ERR_UNSUPPORTED;
   }
 }
