@@ -41,10 +41,6 @@ namespace rfa {
 // The optimum is sharp (head dim 128, S = 8192, 32/8 heads, diagonal / full block: 0 ns 1.57 / 2.99 ms, 50 ns 1.54 / 2.97,
 // 100 ns 1.35 / 2.52, 200 ns 2.13 / 4.20).
 constexpr unsigned kRedSleepNs = 100;
-// Every n-th group of four exponentials of the P^T phase on the FMA pipe (0 = all on the special-function unit, which
-// measured best here: the phase is bound by shared-memory and load/store traffic, not by exp2).
-constexpr int kBwdPolyEvery = 0;
-
 }  // namespace rfa
 
 namespace rfa {
@@ -472,8 +468,6 @@ __global__ void __launch_bounds__(640, 1)
     const int col0 = cw * kHalfCols;
     const uint32_t a_s = tmem_base + lane_addr + Cfg::kTmS + col0;
     const uint32_t a_dp = tmem_base + lane_addr + Cfg::kTmDP + col0;
-    constexpr int kPolyEvery = kBwdPolyEvery;  // of the 8 groups of four exponentials per 32 columns
-    const Exp2Poly exp2_poly;
     const uint64_t nscale2 = pack_f2(-p.scale_log2, -p.scale_log2);
     bool ok = run;
     if (Cfg::kKTmem && run) {
@@ -517,7 +511,9 @@ __global__ void __launch_bounds__(640, 1)
         for (int c = 1; c < NCH; ++c) reg_fence32(r[c]);
         tr.mark(21);
         // P^T = exp2(scale*log2e * S^T - lse2[q]); masked only on diagonal tiles and on a tile that straddles kv_len.
-        // Packed pairs: y = lse2 - c*s in one fma, then 2^(-y); every kPolyEvery-th pair on the FMA pipe.
+        // Packed pairs: y = lse2 - c*s in one fma, then 2^(-y), all on the special-function unit: the phase is bound by
+        // shared-memory and load/store traffic, and a polynomial share costs 2 to 4 % (S 8192, 32/8 heads, diagonal / full:
+        // none 1.50 / 2.88 ms, every 4th group of four 1.53 / 2.92, every 2nd 1.53 / 2.88; S 2048: 120, 121, 123 us).
         auto p_phase = [&](auto mask_tag) {
           constexpr bool kMask = decltype(mask_tag)::value;
 #pragma unroll
@@ -527,19 +523,10 @@ __global__ void __launch_bounds__(640, 1)
               const float4 l4 = *reinterpret_cast<const float4*>(lse2_s + c * 32 + k * 4);
               const uint64_t y01 = fma2(pack_u2(r[c][4 * k + 0], r[c][4 * k + 1]), nscale2, pack_f2(l4.x, l4.y));
               const uint64_t y23 = fma2(pack_u2(r[c][4 * k + 2], r[c][4 * k + 3]), nscale2, pack_f2(l4.z, l4.w));
-              float e0, e1, e2, e3;
-              if (kPolyEvery > 0 && (k % (kPolyEvery > 0 ? kPolyEvery : 1)) == kPolyEvery - 1) {
-                unpack_f2(exp2_poly.neg(y01), e0, e1);
-                unpack_f2(exp2_poly.neg(y23), e2, e3);
-              } else {
-                float y0, y1, y2, y3;
-                unpack_f2(y01, y0, y1);
-                unpack_f2(y23, y2, y3);
-                e0 = fast_exp2(-y0);
-                e1 = fast_exp2(-y1);
-                e2 = fast_exp2(-y2);
-                e3 = fast_exp2(-y3);
-              }
+              float y0, y1, y2, y3;
+              unpack_f2(y01, y0, y1);
+              unpack_f2(y23, y2, y3);
+              float e0 = fast_exp2(-y0), e1 = fast_exp2(-y1), e2 = fast_exp2(-y2), e3 = fast_exp2(-y3);
               if (kMask) {
                 const int qp = q0 + c * 32 + k * 4;
                 if (qp + 0 < mask_lim) e0 = 0.f;

@@ -25,10 +25,12 @@
 
 namespace rfa {
 
-// Every n-th pair of exponentials of the softmax on the FMA pipe (a cubic) instead of the special-function unit,
-// which needs as many cycles per K/V tile as the tensor pipe does; 0 = none.  Diagonal / full block at S = 8192,
-// 32/8 heads, D = 128: every 2nd 0.486 / 0.905 ms, 3rd 0.467 / 0.867, 4th 0.465 / 0.862, 6th 0.469 / 0.866.
-constexpr int kFwdPolyEvery = 4;
+// Every n-th pair of exponentials of the softmax on the FMA pipe (a quartic) instead of the special-function unit, which
+// needs as many cycles per K/V tile as the tensor pipe does; 0 = none.  Diagonal / full block: S 8192, 32/8 heads of 128:
+// every 2nd 553 / 1044 us, 3rd 502 / 953, 4th 510 / 976, none 518 / 991; S 4096, 16 heads of 64: 59.5 / 115.5, 55.5 / 105.3,
+// 55.8 / 106.4, 56.2 / 107.6.  Head dim 256 has one softmax warpgroup to two tiles of tensor work: every 2nd 316 / 574 us,
+// 4th 305 / 559, none 304 / 556.
+constexpr int kFwdPolyEvery = 3;
 
 struct FwdParams {
   float* acc;
@@ -120,7 +122,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
   __shared__ uint64_t bar_kv_empty[kSlots];
   __shared__ uint64_t bar_s_full[NQ * NS];
   constexpr int kPvParts = BN / 32;  // one hand-off per 32 keys
-  constexpr int kPolyEvery = kFwdPolyEvery;  // every n-th pair of exponentials on the FMA pipe (0 = none)
+  constexpr int kPolyEvery = (NQ == 2) ? kFwdPolyEvery : 0;  // every n-th pair of exponentials on the FMA pipe (0 = none)
   __shared__ uint64_t bar_p_ready[NQ * NS * kPvParts];  // [score buffer][part of the keys]
   __shared__ uint64_t bar_pv_done[NQ];
   __shared__ uint32_t tmem_holder;
