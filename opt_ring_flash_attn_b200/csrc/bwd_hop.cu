@@ -35,11 +35,13 @@
 
 namespace rfa {
 
-// Pause (ns) a reduction warp takes after each vector reduction (head dim 256 and the ordered mode; elsewhere the copy
-// engine reduces).  An SM can push 32 B per clock towards the L2; unpaced, the eight reduction warps keep the load/store
-// queue full of reductions and every shared-memory or tensor-memory access of the elementwise warps waits behind them.
-// The optimum is sharp (head dim 128, S = 8192, 32/8 heads, diagonal / full block: 0 ns 1.57 / 2.99 ms, 50 ns 1.54 / 2.97,
-// 100 ns 1.35 / 2.52, 200 ns 2.13 / 4.20).
+// Pause (ns) a reduction warp takes after each vector reduction (head dim 256; up to 128 the copy engine reduces).  An SM
+// can push 32 B per clock towards the L2; unpaced, the eight reduction warps keep the load/store queue full of reductions
+// and every shared-memory or tensor-memory access of the elementwise warps waits behind them.  The optimum is sharp (head
+// dim 128, S = 8192, 32/8 heads, diagonal / full block: 0 ns 1.57 / 2.99 ms, 50 ns 1.54 / 2.97, 100 ns 1.35 / 2.52,
+// 200 ns 2.13 / 4.20).  The ordered mode never pauses: the next K/V tile is waiting for the addition (diagonal / full, paced
+// and not: S 2048, 16/2 heads of 128 177 / 226 -> 164 / 208 us; S 4096, 16 heads of 64 323 / 973 -> 238 / 744; S 8192,
+// 32/8 heads 2.27 / 4.25 -> 2.20 / 3.93 ms).
 constexpr unsigned kRedSleepNs = 100;
 }  // namespace rfa
 
@@ -755,7 +757,7 @@ __global__ void __launch_bounds__(640, 1)
             red_add_v4_f32(base + (c * 8 + k) * 128 + lane * 4, __uint_as_float(r[c][4 * k + 0]) * p.scale,
                            __uint_as_float(r[c][4 * k + 1]) * p.scale, __uint_as_float(r[c][4 * k + 2]) * p.scale,
                            __uint_as_float(r[c][4 * k + 3]) * p.scale);
-            if (kRedSleepNs > 0) __nanosleep(kRedSleepNs);
+            if (order_sem == nullptr) __nanosleep(kRedSleepNs);
           }
         }
         if (order_sem != nullptr) {
