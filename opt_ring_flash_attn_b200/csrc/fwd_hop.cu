@@ -121,7 +121,11 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
   __shared__ uint64_t bar_kv_full[kSlots];
   __shared__ uint64_t bar_kv_empty[kSlots];
   __shared__ uint64_t bar_s_full[NQ * NS];
-  constexpr int kPvParts = BN / 32;  // one hand-off per 32 keys
+  // P is handed over to the issuer in parts: of 32 keys where the product waits for them, of 64 for head dim 64, whose
+  // products take half as long as the softmax (S 16384, 16/4 heads of 64, diagonal / full: 727 / 1423 us in four parts,
+  // 709 / 1385 in two, 709 / 1385 in one; S 8192, 32/8 heads of 128: 508 / 972, 506 / 977, 524 / 1001).
+  constexpr int kPvParts = (DP == 64) ? 2 : 4;
+  constexpr int kPartChunks = BN / 32 / kPvParts;  // chunks of 32 keys per part
   constexpr int kPolyEvery = (NQ == 2) ? kFwdPolyEvery : 0;  // every n-th pair of exponentials on the FMA pipe (0 = none)
   __shared__ uint64_t bar_p_ready[NQ * NS * kPvParts];  // [score buffer][part of the keys]
   __shared__ uint64_t bar_pv_done[NQ];
@@ -311,7 +315,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
             tc_fence_after_sync();
 #pragma unroll
             for (int pc = 0; pc < Cfg::kPieces; ++pc)
-              issue_pv<128, BN, 2 * h, 2 * h + 2>(tmem_base + Cfg::kTmO + pc * 128, s_tm(j), v_lo[pc], idesc_pv,
+              issue_pv<128, BN, 2 * kPartChunks * h, 2 * kPartChunks * (h + 1)>(tmem_base + Cfg::kTmO + pc * 128, s_tm(j), v_lo[pc], idesc_pv,
                                                   (h > 0) || (j > 0) || (p.first == 0), el);
           });
           if (!ok) break;
@@ -365,7 +369,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
                   } else {
                     if (h == 0) tr.mark(11 + 2 * q);
                     tc_fence_after_sync();
-                    issue_pv<DP, BN, 2 * h, 2 * h + 2>(o_tm(q), s_tm(q), v_lo(uv), idesc_pv,
+                    issue_pv<DP, BN, 2 * kPartChunks * h, 2 * kPartChunks * (h + 1)>(o_tm(q), s_tm(q), v_lo(uv), idesc_pv,
                                                        (h > 0) || (j > 0) || (p.first == 0), el);
                   }
                 }
@@ -538,18 +542,18 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
             lp2[i & 1] = add2(lp2[i & 1], p2);
             u[i] = Pack2<T>::pack(p0, p1);
           }
-          if (c > 0) {
-            // the previous 32 keys of P have landed: the issuer may start O += P V on them
+          if (c > 0 && c % kPartChunks == 0) {
+            // the previous part of P has landed: the issuer may start O += P V on them
             tmem_st_wait();
             tc_fence_before_sync();
-            mbar_arrive(&bar_p_ready[(q * NS + sb) * kPvParts + c - 1]);
+            mbar_arrive(&bar_p_ready[(q * NS + sb) * kPvParts + c / kPartChunks - 1]);
           }
           tmem_st16(s_addr + c * 16, u);
           if (c == NCH - 2) tr.mark(24);
         }
         tmem_st_wait();
         tc_fence_before_sync();
-        mbar_arrive(&bar_p_ready[(q * NS + sb) * kPvParts + NCH - 1]);
+        mbar_arrive(&bar_p_ready[(q * NS + sb) * kPvParts + kPvParts - 1]);
         {
           float a0, a1, b0, b1;
           unpack_f2(lp2[0], a0, a1);
