@@ -148,7 +148,7 @@ int rfa_bwd_hop_window(const void* q, const void* k, const void* v, const void* 
 /*
  * rfa_bwd_hop_window with bit-reproducible dQ: the contributions of the K/V tiles to a dQ accumulator tile are
  * added in K/V-tile order (a counter per accumulator tile; each CTA waits, bounded, for the tiles before it), and
- * a GQA group is never split over CTAs.  This restores what the reference's dQ kernel has by construction (it owns
+ * the partial dK/dV of CTAs that share a K/V tile in the order of their runs.  This restores what the reference's dQ kernel has by construction (it owns
  * its tile and updates it with a plain read-modify-write, optimized_ring_flash_attn.py:730-735) and is what
  * `deterministic=True` of the baseline-style wrappers (ring_flash_attn.py:179, 245) selects.  Slower than the
  * unordered hop (CTAs of neighbouring K/V tiles run one query tile apart).
