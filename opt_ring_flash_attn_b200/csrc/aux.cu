@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256) dq_finalize_kernel(const float* __restric
     return;
   }
   __shared__ __align__(16) T tile[128][64 + 8];
-  const int nslice = DP / 64;
+  const int nslice = (D + 63) / 64;
   int idx = blockIdx.x;
   const int slice = idx % nslice; idx /= nslice;
   const int qt = idx % nQt; idx /= nQt;
@@ -346,7 +346,7 @@ int launch_bwd_finish(const float* dq_acc, void* dq, const float* dkdv, void* dk
                       int Hkv, int D, int dtype, cudaStream_t s) {
   const int dp = padded_head_dim(D);
   const int nQt = round_up(Sq, 128) / 128;
-  const unsigned dq_blocks = static_cast<unsigned>(B) * Hq * nQt * (dp / 64);
+  const unsigned dq_blocks = static_cast<unsigned>(B) * Hq * nQt * ceil_div(D, 64);
   const size_t n8 = dkdv ? static_cast<size_t>(B) * Skv * Hkv * D / 8 : 0;
   const unsigned grid = dq_blocks + static_cast<unsigned>((2 * n8 + kCastVec - 1) / kCastVec);
   if (dtype == RFA_DTYPE_BF16)

@@ -292,7 +292,12 @@ __global__ void __launch_bounds__(640, 1)
       if (run) {
         const uint32_t el = elect_one();
         constexpr uint32_t idesc_s = make_idesc(128, BQ, kBf16, false, false);   // K-major x K-major
-        constexpr uint32_t idesc_dv = make_idesc(128, DH, kBf16, false, true);   // A tmem / K-major smem, B MN-major
+        // dV and dK (A from tensor memory / K-major, B MN-major) are as wide as the head dim, not as its padded size (head dim
+        // 256 keeps a constant width: one more live register costs it 2 %).  With dQ^T reduced only by warps that hold
+        // columns of the head dim: B 2, S 1500, 16/4 heads of 96, diagonal / full 71.4 / 116 -> 66.2 / 106 us; S 4096, 16 heads
+        // of 32 130 / 257 -> 125 / 246; B 2, S 4096, 16 heads of 160 1166 / 1935 -> 1126 / 1898.  S^T and dP^T do run over
+        // the padding: a predicate per step costs the issuer more (25 % at head dim 256) than the steps it saves.
+        const uint32_t idesc_dv = make_idesc(128, DP > 128 ? DH : min((p.D + 15) / 16 * 16, DH), kBf16, false, true);
         constexpr uint32_t idesc_dq = make_idesc(128, BQ, kBf16, true, true);    // both MN-major
         const uint32_t tm_s = tmem_base + Cfg::kTmS;
         const uint32_t tm_dp = tmem_base + Cfg::kTmDP;
@@ -682,7 +687,17 @@ __global__ void __launch_bounds__(640, 1)
     const int quarter = warp & 3;
     const int drow = quarter * 32 + lane;  // row of dQ^T = head-dim index inside this CTA's half
     const int d = hf * DH + drow;
-    const bool d_ok = (drow < DH);
+    const bool d_ok = (drow < DH) && (hf * DH + quarter * 32 < p.D);  // the same for the whole warp
+    // Warps with nothing but padding in their rows only take part in releasing the columns: in a loop of their own, except
+    // at head dim 64, where half of the warps have no rows at all (143 us inside the common loop, 147 apart: S 4096, 16
+    // heads; head dim 128 spills fewer registers with it apart).
+    constexpr bool kApart = (DP > 64);
+    if (kApart && !d_ok) {
+      for (int t = 0; t < T_total && run; ++t) {
+        if (!mbar_wait_warp(&bar_dq_full, t & 1, abort_p)) break;
+        mbar_arrive(&bar_dq_drained);
+      }
+    }
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t a_dq = tmem_base + lane_addr + Cfg::kTmDQ + half * kRedCols;
     // dQ accumulator layout (fp32, private): [b][hq][Spad/128 tiles][DP/32][32 groups of 4 rows][32][4].  Lane = head-dim
@@ -690,7 +705,7 @@ __global__ void __launch_bounds__(640, 1)
     // what a warp adds for a tile is one contiguous run.
     constexpr size_t kTileElems = static_cast<size_t>(128) * DP;
     const int nQt128 = p.Spad / 128;
-    bool ok = run;
+    bool ok = run && (!kApart || d_ok);
     for (int t = 0; t < T_total && ok; ++t) {
       const int hq = q_head(t);
       const int q0 = q_tile(t) * BQ;
@@ -701,7 +716,7 @@ __global__ void __launch_bounds__(640, 1)
       float* base = p.dq_acc + ((static_cast<size_t>(b) * p.Hq + hq) * nQt128 + q0 / 128) * kTileElems +
                     (d / 32) * 4096 + (q0 % 128 + half * kRedCols) / 4 * 128;  // of the warp's 32 head-dim columns
       uint32_t r[NCR][32];
-      if (d_ok) {
+      if (kApart || d_ok) {
 #pragma unroll
         for (int c = 0; c < NCR; ++c) tmem_ld32(a_dq + c * 32, r[c]);
         tmem_ld_wait32(r[0]);
@@ -723,32 +738,31 @@ __global__ void __launch_bounds__(640, 1)
                     quarter;
         if (!wait_count(order_sem, kvt, lane == 0 && d_ok, abort_p)) { ok = false; break; }
       }
+      if (!kApart && !d_ok) continue;
       if (Cfg::kStageDQ && order_sem == nullptr) {
-        if (d_ok) {
-          constexpr int kChunks = kRedCols / 4 / Cfg::kDQGroups;
-          const uint32_t wbuf = ((half * (Cfg::kDQWarps / 2) + quarter) * 2) * Cfg::kDQBufBytes;
-          static_for<0, kChunks>([&](auto ck_) {
-            constexpr int ck = decltype(ck_)::value;
-            const uint32_t buf = wbuf + ((kChunks % 2 == 0) ? (ck & 1) : (t & 1)) * Cfg::kDQBufBytes;
-            float4* stage = reinterpret_cast<float4*>(dq_ptr + buf) + lane;
-            if (lane == 0) bulk_wait_read<1>();  // the reduction before the last one has read this buffer
-            __syncwarp();
+        constexpr int kChunks = kRedCols / 4 / Cfg::kDQGroups;
+        const uint32_t wbuf = ((half * (Cfg::kDQWarps / 2) + quarter) * 2) * Cfg::kDQBufBytes;
+        static_for<0, kChunks>([&](auto ck_) {
+          constexpr int ck = decltype(ck_)::value;
+          const uint32_t buf = wbuf + ((kChunks % 2 == 0) ? (ck & 1) : (t & 1)) * Cfg::kDQBufBytes;
+          float4* stage = reinterpret_cast<float4*>(dq_ptr + buf) + lane;
+          if (lane == 0) bulk_wait_read<1>();  // the reduction before the last one has read this buffer
+          __syncwarp();
 #pragma unroll
-            for (int k = 0; k < Cfg::kDQGroups; ++k) {
-              constexpr int g0 = ck * Cfg::kDQGroups;
-              const uint32_t* v = &r[(g0 + k) / 8][((g0 + k) % 8) * 4];
-              stage[k * 32] = make_float4(__uint_as_float(v[0]) * p.scale, __uint_as_float(v[1]) * p.scale,
-                                          __uint_as_float(v[2]) * p.scale, __uint_as_float(v[3]) * p.scale);
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              bulk_reduce_add_f32(base + ck * Cfg::kDQGroups * 128, smem_base + Cfg::kOffDQ + buf, Cfg::kDQBufBytes);
-              bulk_commit();
-            }
-          });
-        }
-      } else if (d_ok) {
+          for (int k = 0; k < Cfg::kDQGroups; ++k) {
+            constexpr int g0 = ck * Cfg::kDQGroups;
+            const uint32_t* v = &r[(g0 + k) / 8][((g0 + k) % 8) * 4];
+            stage[k * 32] = make_float4(__uint_as_float(v[0]) * p.scale, __uint_as_float(v[1]) * p.scale,
+                                        __uint_as_float(v[2]) * p.scale, __uint_as_float(v[3]) * p.scale);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            bulk_reduce_add_f32(base + ck * Cfg::kDQGroups * 128, smem_base + Cfg::kOffDQ + buf, Cfg::kDQBufBytes);
+            bulk_commit();
+          }
+        });
+      } else {
         // rows beyond Sq and head-dim columns beyond D hold exact zeros (zero-filled operands, P = 0)
 #pragma unroll
         for (int c = 0; c < NCR; ++c) {

@@ -270,10 +270,11 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
       // The whole warp runs this loop converged; the elected lane issues.  A commit makes its mbarrier track every MMA
       // issued before it, so the arrival on bar_s_full for tile j+1 also tells the softmax warps that O += P_j V_j has
       // retired; bar_pv_done is only needed after the last tile.
+      const uint32_t el = elect_one();
+      const int d16 = (p.D + 15) / 16 * 16;  // O is as wide as the head dim (96 instead of 128 columns: -2 %, 160 instead of 256: -3 %)
       if constexpr (NS == 2) {
-        const uint32_t el = elect_one();
         constexpr uint32_t idesc_qk = make_idesc(128, BN, kBf16, false, false);
-        constexpr uint32_t idesc_pv = make_idesc(128, 128, kBf16, false, true);
+        auto idesc_pv = [&](int pc) { return make_idesc(128, min(d16 - pc * 128, 128), kBf16, false, true); };
         const uint32_t q_lo = desc_lo_kmajor(s_q);
         SlotWalk<kSlots> w;
         auto s_tm = [&](int j) { return tmem_base + Cfg::kTmS + (j & 1) * BN; };
@@ -315,7 +316,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
             tc_fence_after_sync();
 #pragma unroll
             for (int pc = 0; pc < Cfg::kPieces; ++pc)
-              issue_pv<128, BN, 2 * kPartChunks * h, 2 * kPartChunks * (h + 1)>(tmem_base + Cfg::kTmO + pc * 128, s_tm(j), v_lo[pc], idesc_pv,
+              issue_pv<128, BN, 2 * kPartChunks * h, 2 * kPartChunks * (h + 1)>(tmem_base + Cfg::kTmO + pc * 128, s_tm(j), v_lo[pc], idesc_pv(pc),
                                                   (h > 0) || (j > 0) || (p.first == 0), el);
           });
           if (!ok) break;
@@ -325,9 +326,8 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
           tr.mark(12);
         }
       } else {
-        const uint32_t el = elect_one();
         constexpr uint32_t idesc_qk = make_idesc(128, BN, kBf16, false, false);
-        constexpr uint32_t idesc_pv = make_idesc(128, DP, kBf16, false, true);
+        const uint32_t idesc_pv = make_idesc(128, d16, kBf16, false, true);
         auto slot_of = [&](int u) { return u % kSlots; };
         auto par_of = [&](int u) { return static_cast<uint32_t>((u / kSlots) & 1); };
         // descriptor low words of the operand tiles (K: K-major, V: MN-major, Q: K-major)
@@ -403,6 +403,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
     // selected, not indexed: an array indexed at run time would live in local memory for the issuer as well
     const int n = (NQ == 2 && q == 1) ? ntile[NQ - 1] : ntile[0];
     const int m0_q = (NQ == 2 && q == 1) ? m0[NQ - 1] : m0[0];
+    const int n_c32 = (p.D + 31) / 32;  // chunks of O that hold columns of the head dim
     const int row_g = m0_q + row;  // local query position
     const uint32_t o_addr = tmem_base + lane_addr + Cfg::kTmO + q * DP;
     const int qt = tq0 + qs * NQ + q;
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
         m_used = p.m[ml_idx];
         l_sum = p.l[ml_idx];
 #pragma unroll 1
-        for (int c = 0; c < DP / 32; ++c) {
+        for (int c = 0; c < n_c32; ++c) {
           uint32_t r[32];
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
@@ -503,7 +504,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
             tc_fence_after_sync();
           }
 #pragma unroll 1
-          for (int c = 0; c < DP / 16; ++c) {
+          for (int c = 0; c < 2 * n_c32; ++c) {
             uint32_t o16[16];
             tmem_ld16(o_addr + c * 16, o16);
             tmem_ld_wait16(o16);
@@ -575,7 +576,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
           const bool row_ok = row_g < p.Sq;
           T* orow = reinterpret_cast<T*>(p.out) + ((static_cast<size_t>(b) * p.Sq + row_g) * p.Hq + h) * p.D;
 #pragma unroll 1
-          for (int c = 0; c < DP / 32; ++c) {
+          for (int c = 0; c < n_c32; ++c) {
             uint32_t r[32];
             tmem_ld32(o_addr + c * 32, r);
             tmem_ld_wait32(r);
@@ -596,7 +597,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
           if (row_ok) p.lse[ml_idx] = (m_used + log2f(l_sum)) * 0.6931471805599453f;
         } else {
 #pragma unroll 1
-          for (int c = 0; c < DP / 32; ++c) {
+          for (int c = 0; c < n_c32; ++c) {
             uint32_t r[32];
             tmem_ld32(o_addr + c * 32, r);
             tmem_ld_wait32(r);
