@@ -44,6 +44,9 @@ int bwd_check_args(const void* q, const void* k, const void* v, const void* dout
 // Measured, hop kernel alone, unsplit / chosen (chosen split; the neighbours are slower):
 //   S 2048, 32/8 heads of 128, diagonal 183 / 108 us (2: 109, 3: 130);  16/2 heads, diagonal 344 / 66 (8: 66, 6: 74),
 //   full 348 / 101 (4);  B 2, S 1500, 16/4 heads of 96: 137 / 72 (3), full 140 / 109 (3);  S 1024, 32 heads: 49 (1).
+// Two runs may be as short as two tiles (S 512, 8 heads of 128, diagonal / full: 21.5 / 21.6 us unsplit, 18.5 / 18.6 in two).
+// An overhead of 2 or 3 tiles instead of 2.5 gains 7 % in places and loses as much in others (3: S 4096, 32/4 heads, diagonal
+// 404 -> 385 us, B 2, S 1500, 16/4 heads of 96 65.8 -> 70.6).
 inline void choose_split(BwdParams& pr, long long base_units, int bq) {
   constexpr int kSMs = 148;
   constexpr double kCtaOverhead = 2.5;
@@ -69,7 +72,7 @@ inline void choose_split(BwdParams& pr, long long base_units, int bq) {
                          static_cast<long long>(pr.Hkv) * n_kv <= static_cast<long long>(pr.Hq) * ceil_div(pr.Sq, 128);
   int best = 1;
   double best_t = 0;
-  for (int ns = 1; ns <= kMaxSplit && (ns == 1 || heaviest >= kMinRun * ns); ++ns) {
+  for (int ns = 1; ns <= kMaxSplit && (ns == 1 || heaviest >= (ns == 2 ? 2 : kMinRun) * ns); ++ns) {
     const double n = static_cast<double>(base_units) * ns;
     const double longest = heaviest / ns + kCtaOverhead;
     double t;
