@@ -30,7 +30,9 @@ def _deterministic_now() -> bool:
 def deterministic(enabled: bool = True):
     """Calls of :func:`ring_flash_attn` made inside this context compute bit-reproducible gradients: the dQ
     contributions of the K/V tiles are added in a fixed order instead of by unordered fp32 reductions (the
-    reference's dQ kernel is deterministic by construction, optimized_ring_flash_attn.py:730-735).  The choice is
+    reference's dQ kernel is deterministic by construction, optimized_ring_flash_attn.py:730-735), and so are the parts of
+    dK and dV of a K/V tile that several thread blocks share.  Outside it dQ varies in its last bits from call to call, and
+    so may dK and dV of calls with fewer K/V heads than query heads; those of calls with as many do not.  The choice is
     taken at forward time and holds for that call's backward.  ``RFA_B200_DETERMINISTIC=1`` sets the default."""
     prev = getattr(_mode, "deterministic", None)
     _mode.deterministic = enabled

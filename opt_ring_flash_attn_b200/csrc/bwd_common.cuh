@@ -47,6 +47,10 @@ int bwd_check_args(const void* q, const void* k, const void* v, const void* dout
 // Two runs may be as short as two tiles (S 512, 8 heads of 128, diagonal / full: 21.5 / 21.6 us unsplit, 18.5 / 18.6 in two).
 // An overhead of 2 or 3 tiles instead of 2.5 gains 7 % in places and loses as much in others (3: S 4096, 32/4 heads, diagonal
 // 404 -> 385 us, B 2, S 1500, 16/4 heads of 96 65.8 -> 70.6).
+// Without head groups (MHA) dK and dV keep the same bits from call to call, ordered mode or not: two runs may be added to
+// the cleared buffer in either order, three, or two and the previous partial sums, may not.  This matters below some four
+// heads (hop alone, any split / at most two: S 8192, 1 head of 128, diagonal 59 / 86 us; S 4096, 1 head of 64, diagonal / full
+// 24.6, 26.7 / 39.4, 41.0; S 2048, 4 heads of 128 34.8, 34.8 / 32.8, 34.9), where the host takes longer than the kernels.
 inline void choose_split(BwdParams& pr, long long base_units, int bq) {
   constexpr int kSMs = 148;
   constexpr double kCtaOverhead = 2.5;
@@ -70,9 +74,10 @@ inline void choose_split(BwdParams& pr, long long base_units, int bq) {
   // the ordered mode has counters for as many K/V tiles as there are query tiles of 128 rows
   const bool may_split = pr.dq_order == nullptr ||
                          static_cast<long long>(pr.Hkv) * n_kv <= static_cast<long long>(pr.Hq) * ceil_div(pr.Sq, 128);
+  const int max_split = !may_split ? 1 : (G > 1 || pr.dq_order != nullptr) ? kMaxSplit : pr.accumulate_prev ? 1 : 2;
   int best = 1;
   double best_t = 0;
-  for (int ns = 1; ns <= kMaxSplit && (ns == 1 || heaviest >= (ns == 2 ? 2 : kMinRun) * ns); ++ns) {
+  for (int ns = 1; ns <= max_split && (ns == 1 || heaviest >= (ns == 2 ? 2 : kMinRun) * ns); ++ns) {
     const double n = static_cast<double>(base_units) * ns;
     const double longest = heaviest / ns + kCtaOverhead;
     double t;
@@ -84,7 +89,6 @@ inline void choose_split(BwdParams& pr, long long base_units, int bq) {
       t = load > longest ? load : longest;
     }
     if (ns == 1 || t < best_t * kSplitGain) { best = ns; best_t = t; }
-    if (!may_split) break;
   }
   pr.nsplit = best;
   pr.reduce_out = best > 1 ? 1 : 0;
