@@ -474,28 +474,30 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
           mxp[c][1] = __uint_as_float(r[c][1]);
 #pragma unroll
           for (int i = 2; i < 30; i += 4) {
-            mxp[c][0] = max3(mxp[c][0], __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
-            mxp[c][1] = max3(mxp[c][1], __uint_as_float(r[c][i + 2]), __uint_as_float(r[c][i + 3]));
+            mxp[c][0] = max3_nan(mxp[c][0], __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
+            mxp[c][1] = max3_nan(mxp[c][1], __uint_as_float(r[c][i + 2]), __uint_as_float(r[c][i + 3]));
           }
-          mxp[c][0] = max3(mxp[c][0], __uint_as_float(r[c][30]), __uint_as_float(r[c][31]));
+          mxp[c][0] = max3_nan(mxp[c][0], __uint_as_float(r[c][30]), __uint_as_float(r[c][31]));
         }
-        float mx = fmaxf(mxp[0][0], mxp[0][1]);
+        float mx = max_nan(mxp[0][0], mxp[0][1]);
 #pragma unroll
-        for (int c = 1; c < NCH; ++c) mx = fmaxf(mx, fmaxf(mxp[c][0], mxp[c][1]));
-        const float m_new = fmaxf(m_used, mx * p.scale_log2);
+        for (int c = 1; c < NCH; ++c) mx = max3_nan(mx, mxp[c][0], mxp[c][1]);
+        const float m_new = max_nan(m_used, mx * p.scale_log2);
         tr.mark(21);
 
-        // lazy rescale: only when the maximum grew by more than 2^8
+        // lazy rescale: only when the maximum grew by more than 2^8, or is no number.  A NaN or infinite score makes its
+        // row NaN through the maximum (here, or in the epilogue where it stood in the only tile): the polynomial would
+        // turn the exponential of a NaN into 2^-125.
         bool need;
         if (j == 0 && p.first) {
           m_used = m_new;
           need = false;
         } else {
-          need = (m_new - m_used) > 8.0f;
+          need = !(m_new - m_used <= 8.0f);
         }
         if (__any_sync(0xffffffffu, need)) {
           const float alpha = need ? fast_exp2(m_used - m_new) : 1.0f;
-          if (need) m_used = m_new;
+          if (need) m_used = m_new + (m_new - m_new);
           l_sum *= alpha;
           // With one score buffer the arrival on bar_s_full that let this iteration start was committed after
           // O += P_{j-1} V_{j-1} was issued, so that product has retired; with two buffers it has its own barrier.
@@ -571,6 +573,7 @@ __global__ void __launch_bounds__(128 + NQ * 128, 1)
       if (ok) ok = mbar_wait_warp(&bar_pv_done[q], (NS == 2) ? ((n - 1) & 1) : 0, abort_p);
       if (ok) {
         tc_fence_after_sync();
+        l_sum += m_used - m_used;  // nothing, or NaN
         if (last_here) {
           const float inv = 1.0f / l_sum;
           const bool row_ok = row_g < p.Sq;

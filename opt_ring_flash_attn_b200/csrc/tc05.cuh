@@ -544,10 +544,15 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// Largest of three (one instruction on sm_100; the non-NaN operand wins, as with fmaxf).
-__device__ __forceinline__ float max3(float a, float b, float c) {
+// Largest of two or three (one instruction on sm_100); NaN if any of them is.
+__device__ __forceinline__ float max_nan(float a, float b) {
   float y;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
   return y;
 }
 
@@ -590,7 +595,7 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 }
 // 2^x for a pair, on the FMA pipe instead of the special-function unit: x = n + f with n = round(x) (magic-number
 // rounding), 2^f by a quartic on [-0.5, 0.5] (minimax, relative error 2.7e-6 in fp32), and n added to the exponent field.
-// x is clamped to >= -125 so that masked (-inf) entries come out as ~2^-125.
+// x is clamped to >= -125 so that masked (-inf) entries come out as ~2^-125; so does a NaN: the caller looks for those.
 struct Exp2Poly {
   uint64_t magic, c0, c1, c2, c3, c4;
   __device__ __forceinline__ Exp2Poly() {
