@@ -311,6 +311,14 @@ class HopRecorder:
         self._n = native
         self.events = []  # (name, start event, end event)
 
+    def bwd_local(self, q, k, v, out, dout, lse, delta, lse2, dq_acc, dkdv, dq, dk, dv, scale, causal, status, dq_order=None):
+        """The backward without a ring is one call of three kernels: here its parts, so that the hop has a row of its own."""
+        self.bwd_prepare(out, dout, lse, delta, lse2, dq_acc, status)
+        self.bwd_hop(q, k, v, dout, lse2, delta, dq_acc, None, dkdv, scale, False, causal, status, dq_order=dq_order)
+        self.dq_finalize(dq_acc, dq)
+        self.cast_from_f32(dkdv[0], dk)
+        self.cast_from_f32(dkdv[1], dv)
+
     def __getattr__(self, name):
         fn = getattr(self._n, name)
         if not callable(fn) or name.startswith("_"):

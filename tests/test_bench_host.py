@@ -48,3 +48,36 @@ def test_timeline_summary():
     assert abs(s["hop_kernel_ms"] - 2.9) < 1e-9 and abs(s["accumulate_ms"] - 0.04) < 1e-9
     assert abs(s["other_kernel_ms"] - 0.08) < 1e-9 and abs(s["kernel_ms"] - 3.02) < 1e-9
     assert s["exposed_wait_ms"] == {"fwd_kv": 0.003, "bwd_kv": 0, "bwd_dkdv": 0.2}
+
+
+def test_timeline_without_a_ring_has_a_row_for_every_hop(monkeypatch):
+    """The schedules run the backward of a single shard in one call; the recorder times its parts."""
+    import fake_kernels
+    import torch
+
+    from opt_ring_flash_attn_b200 import schedule
+
+    class Event:
+        def __init__(self, enable_timing=False):
+            pass
+
+        def record(self):
+            pass
+
+    class Native:
+        def __getattr__(self, name):
+            return getattr(fake_kernels, name)
+
+        def bwd_local(self, *a, **kw):
+            raise AssertionError("one call, nothing to time inside it")
+
+    b = _bench()
+    monkeypatch.setattr(b.torch.cuda, "Event", Event)
+    rec = b.HopRecorder(Native())
+    q, k, v, dout = (torch.randn(1, 64, 2, 16).bfloat16() for _ in range(4))
+    out, lse = schedule.ring_forward(None, q, k, v, 0.25, True, kernels=rec)
+    grads = schedule.ring_backward(None, dout, q, k, v, out, lse, 0.25, True, kernels=rec)
+    assert [name for name, _, _ in rec.events] == ["fwd_hop", "bwd_prepare", "bwd_hop", "dq_finalize", "cast_from_f32",
+                                                   "cast_from_f32"]
+    for t, g in zip((q, k, v), grads):
+        assert g.shape == t.shape and torch.isfinite(g.float()).all()
