@@ -148,18 +148,8 @@ def _local_backward(kn, group, dout, q, k, v, out, lse, softmax_scale: float, ca
     workspace.raise_if_failed(ws, "ring_flash_attn backward")
     dout = dout.contiguous()
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    order = ws.dq_order if deterministic else None
-    if hasattr(kn, "bwd_local"):
-        kn.bwd_local(q, k, v, out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.dkdv[0], dq, dk, dv, softmax_scale,
-                     causal, ws.status, dq_order=order)
-    else:  # a kernel backend that only has the parts
-        buf = ws.dkdv[0]
-        kn.bwd_prepare(out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.status)
-        kn.bwd_hop(q, k, v, dout, ws.lse2, ws.delta, ws.dq_acc, None, buf, softmax_scale, False, causal, ws.status,
-                   dq_order=order)
-        kn.dq_finalize(ws.dq_acc, dq)
-        kn.cast_from_f32(buf[0], dk)
-        kn.cast_from_f32(buf[1], dv)
+    kn.bwd_local(q, k, v, out, dout, lse, ws.delta, ws.lse2, ws.dq_acc, ws.dkdv[0], dq, dk, dv, softmax_scale, causal,
+                 ws.status, dq_order=ws.dq_order if deterministic else None)
     workspace.publish_status(ws, "ring_flash_attn backward")
     return dq, dk, dv
 

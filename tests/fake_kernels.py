@@ -125,3 +125,12 @@ def dkdv_accumulate_to16(prev, block, out, stream=None):
 
 def cast_from_f32(src, dst, stream=None):
     dst.copy_(src.to(dst.dtype))
+
+
+def bwd_local(q, k, v, out, dout, lse, delta, lse2, dq_acc, dkdv, dq, dk, dv, scale, causal, status, stream=None,
+              dq_order=None):
+    bwd_prepare(out, dout, lse, delta, lse2, dq_acc, status)
+    bwd_hop(q, k, v, dout, lse2, delta, dq_acc, None, dkdv, scale, False, causal, status, dq_order=dq_order)
+    dq_finalize(dq_acc, dq)
+    cast_from_f32(dkdv[0], dk)
+    cast_from_f32(dkdv[1], dv)

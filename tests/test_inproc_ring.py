@@ -30,6 +30,32 @@ def test_contiguous_schedule_in_process(W, causal, Hq, Hkv, wire16, monkeypatch)
         assert _rel(dvs[r], ref["dv"][r]) <= 2e-2
 
 
+@pytest.mark.parametrize("causal,deterministic", [(True, False), (False, True)])
+def test_single_shard_runs_its_backward_in_one_call(causal, deterministic):
+    import fake_kernels
+    from opt_ring_flash_attn_b200 import schedule
+
+    calls = []
+
+    class Kernels:
+        def __getattr__(self, name):
+            def call(*a, **kw):
+                calls.append((name, kw.get("dq_order") is not None))
+                return getattr(fake_kernels, name)(*a, **kw)
+
+            return call
+
+    q, k, v, dout = make_inputs(52, 1, 96, 4, 2, 32, dtype=torch.bfloat16)
+    out, lse = schedule.ring_forward(None, q, k, v, 0.3, causal, kernels=Kernels())
+    grads = schedule.ring_backward(None, dout, q, k, v, out, lse, 0.3, causal, kernels=Kernels(),
+                                   deterministic=deterministic)
+    assert calls == [("fwd_hop", False), ("bwd_local", deterministic)]
+    ref = ring_attn_oracle([q], [k], [v], [dout], causal=causal, softmax_scale=0.3)
+    assert (out.float() - ref["out"][0]).abs().max().item() <= 1e-2
+    for g, name in zip(grads, ("dq", "dk", "dv")):
+        assert _rel(g, ref[name][0]) <= 2e-2
+
+
 def test_zigzag_schedule_in_process():
     import fake_kernels
     from inproc_ring import run_ring
