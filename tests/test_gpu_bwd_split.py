@@ -1,5 +1,5 @@
-"""K/V tiles of the backward hop shared by several CTAs: runs that cross head boundaries, do not divide evenly, or start
-inside a window, and the ordered mode (bit-reproducible with any split)."""
+"""K/V tiles of the backward hop shared by several CTAs: runs that cross head boundaries or do not divide evenly, the ordered
+mode (bit-reproducible with any split), and what repeats without it.  Windows: test_gpu_bwd_windows.py."""
 import pytest
 import torch
 

@@ -8,16 +8,17 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("D", [8, 16, 24, 40, 56, 72, 88, 104, 120, 136, 152, 168, 200, 248])
+@pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("ordered", [False, True])
-def test_every_width_of_the_last_step(D, ordered):
+def test_every_width_of_the_last_step(D, ordered, causal):
     import opt_ring_flash_attn_b200 as rfa
 
     q, k, v, dout = (x.cuda() for x in make_inputs(D, 1, 300, 4, 2, D, dtype=torch.bfloat16))
     leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
     with rfa.deterministic(ordered):
-        out, lse = rfa.ring_flash_attn_with_lse(*leaves, causal=not ordered)
+        out, lse = rfa.ring_flash_attn_with_lse(*leaves, causal=causal)
     grads = torch.autograd.grad(out, leaves, dout)
-    ref = ring_attn_oracle([q], [k], [v], [dout], causal=not ordered)
+    ref = ring_attn_oracle([q], [k], [v], [dout], causal=causal)
     assert (lse - ref["lse"][0]).abs().max().item() <= 1e-3
     # the parity tests' bounds: P, dS and the results are rounded to bf16
     assert (out.float() - ref["out"][0]).abs().max().item() <= 1e-2 * max(1.0, ref["out"][0].abs().max().item())

@@ -154,7 +154,8 @@ def test_long_context_distribution():
 
 def test_epilogue_accumulate_path():
     """The backward kernel's own `dkdv_out = dkdv_prev + block` epilogue (accumulate_prev=1), which the product
-    schedule replaces by a separate accumulate kernel: a three-rank walk written out by hand."""
+    schedule replaces by a separate accumulate kernel: a three-rank walk written out by hand.  Both shapes share their
+    K/V tiles among CTAs, which add to the buffer in place; tests/test_gpu_bwd_accumulate.py has the other routes."""
     run_case(1, 384, 4, 2, 128, 3, True, seed=3, path="emulator")
     run_case(1, 200, 2, 2, 256, 2, False, seed=5, path="emulator")
 
