@@ -146,12 +146,13 @@ int rfa_bwd_hop_window(const void* q, const void* k, const void* v, const void* 
                        int causal_diag, int q_begin, int kv_len, int* status, void* stream);
 
 /*
- * rfa_bwd_hop_window with bit-reproducible dQ: the contributions of the K/V tiles to a dQ accumulator tile are
+ * rfa_bwd_hop_window with bit-reproducible results: the contributions of the K/V tiles to a dQ accumulator tile are
  * added in K/V-tile order (a counter per accumulator tile; each CTA waits, bounded, for the tiles before it), and
- * the partial dK/dV of CTAs that share a K/V tile in the order of their runs.  This restores what the reference's dQ kernel has by construction (it owns
- * its tile and updates it with a plain read-modify-write, optimized_ring_flash_attn.py:730-735) and is what
- * `deterministic=True` of the baseline-style wrappers (ring_flash_attn.py:179, 245) selects.  Slower than the
- * unordered hop (CTAs of neighbouring K/V tiles run one query tile apart).
+ * the partial dK/dV of CTAs that share a K/V tile in the order of their runs.  This restores what the reference's dQ
+ * kernel has by construction (it owns its tile and updates it with a plain read-modify-write,
+ * optimized_ring_flash_attn.py:730-735) and is what `deterministic=True` of the baseline-style wrappers
+ * (ring_flash_attn.py:179, 245) selects.  Slower than the unordered hop (CTAs of neighbouring K/V tiles run one query
+ * tile apart), whose dQ varies in its last bits from call to call, as dK and dV may where Hq > Hkv.
  *  dq_order  int32 [rfa_dq_order_elems(B,Sq,Hq,D)] scratch, cleared by the call itself.
  */
 size_t rfa_dq_order_elems(int B, int Sq, int Hq, int D);

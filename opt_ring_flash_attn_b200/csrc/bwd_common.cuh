@@ -41,10 +41,13 @@ int bwd_check_args(const void* q, const void* k, const void* v, const void* dout
 // K/V tile to several CTAs, whose partial dK/dV are added with vector reductions into a prepared buffer.
 // Picks the split with the shortest estimated makespan, a larger one only for a gain of 5 %; runs shorter than three
 // tiles cost more in reductions than they save (S = 256, 8 heads of 64: 14.3 us unsplit, 15.3 us in two).
-// Measured, hop kernel alone, unsplit / chosen (chosen split; the neighbours are slower):
-//   S 2048, 32/8 heads of 128, diagonal 183 / 108 us (2: 109, 3: 130);  16/2 heads, diagonal 344 / 66 (8: 66, 6: 74),
-//   full 348 / 101 (4);  B 2, S 1500, 16/4 heads of 96: 137 / 72 (3), full 140 / 109 (3);  S 1024, 32 heads: 49 (1).
-// Two runs may be as short as two tiles (S 512, 8 heads of 128, diagonal / full: 21.5 / 21.6 us unsplit, 18.5 / 18.6 in two).
+// Measured, hop alone with the clearing of its buffer, unsplit / chosen (chosen split; neighbours), us:
+//   S 2048, 32/8 heads of 128, diagonal 161 / 99 (2; 3: 114), full 179 (1; 2: 197);  16/2 heads, diagonal 291 / 60 (7; 6: 65,
+//   8: 60), full 294 / 92 (4; 3: 114, 8: 99);  B 2, S 1500, 16/4 heads of 96, diagonal 120 / 64 (3; 2: 67, 4: 74), full
+//   118 / 95 (3; 2: 128, 4: 113);  S 1024, 32 heads of 128, diagonal / full 45 / 63 (1; 2: 72 / 88).
+// Two runs may be as short as two tiles, which gains up to 5 % at head dim 64 and 5 to 16 % above (unsplit / in two, us, full:
+// S 512, 8 heads of 128 21.5 / 18.5, of 64 15.2 / 14.4, 16 heads of 128 21.7 / 20.5; S 256, 16/8 heads of 128 21.2 / 18.5, 8 heads
+// of 256 20.8 / 18.5; S 128, 32/8 heads of 128 21.1 / 18.5; B 2, S 250, 4 heads of 160 20.1 / 17.7; S 600, 8 heads 23.8 / 20.5).
 // An overhead of 2 or 3 tiles instead of 2.5 gains 7 % in places and loses as much in others (3: S 4096, 32/4 heads, diagonal
 // 404 -> 385 us, B 2, S 1500, 16/4 heads of 96 65.8 -> 70.6).
 // Without head groups (MHA) dK and dV keep the same bits from call to call, ordered mode or not: two runs may be added to

@@ -1,6 +1,6 @@
 // Backward ring hop against one K/V block.  One CTA owns a 128-row K/V tile of
 // one kv head and walks over every query head of its GQA group and every query
-// tile that can see it.  Five tensor-core products per (kv tile, q tile) pair,
+// tile that can see it, or over one of several equal runs of them (choose_split).  Five tensor-core products per (kv tile, q tile) pair,
 // all computed in the transposed orientation so that the kv row is the TMEM
 // lane and the accumulators dK, dV stay resident in tensor memory:
 //   S^T  = K Q^T                (smem x smem)      -> P^T = exp2(scale*S^T - lse2[q])
@@ -37,16 +37,14 @@ namespace rfa {
 
 // Pause (ns) a reduction warp takes after each vector reduction (head dim 256; up to 128 the copy engine reduces).  An SM
 // can push 32 B per clock towards the L2; unpaced, the eight reduction warps keep the load/store queue full of reductions
-// and every shared-memory or tensor-memory access of the elementwise warps waits behind them.  The optimum is sharp (head
-// dim 128, S = 8192, 32/8 heads, diagonal / full block: 0 ns 1.57 / 2.99 ms, 50 ns 1.54 / 2.97, 100 ns 1.35 / 2.52,
-// 200 ns 2.13 / 4.20).  The ordered mode never pauses: the next K/V tile is waiting for the addition (diagonal / full, paced
-// and not: S 2048, 16/2 heads of 128 177 / 226 -> 164 / 208 us; S 4096, 16 heads of 64 323 / 973 -> 238 / 744; S 8192,
-// 32/8 heads 2.27 / 4.25 -> 2.20 / 3.93 ms).
+// and every shared-memory or tensor-memory access of the elementwise warps waits behind them.  The optimum is sharp (150 ns
+// behaves like 200; 0 / 20 / 50 / 100 / 150 / 200 ns, hop alone, us: B 2, S 4096, 16 heads of 256, full
+// 2297 / 2197 / 2177 / 1990 / 2288 / 2288; 16 heads of 160, diagonal 1143 / 1121 / 1121 / 1085 / 1241 / 1240, full 1980 /
+// 1934 / 1920 / 1790 / 2250 / 2250; S 700, 16 heads of 256, full 73.8 / 71.7 / 71.7 / 69.7 / 75.8 / 75.8).  The ordered mode
+// never pauses: the next K/V tile is waiting for the addition (head dims up to 128, diagonal / full, paced and not: S 2048,
+// 16/2 heads of 128 177 / 226 -> 164 / 208 us; S 4096, 16 heads of 64 323 / 973 -> 238 / 744; S 8192, 32/8 heads
+// 2.27 / 4.25 -> 2.20 / 3.93 ms).
 constexpr unsigned kRedSleepNs = 100;
-}  // namespace rfa
-
-namespace rfa {
-
 
 // Bounded wait of one lane until a counter in global memory has reached `target`; the whole warp gets the answer
 // (false: the CTA is aborting).
@@ -90,7 +88,8 @@ struct BwdCfg {
   // (paced 100 ns) / 300 us (20 ns), bulk reductions 291.  At head dim 128 the 32 KB come from the second dO stage (dO of
   // the next tile is wanted after dQ^T has been drained, some 2500 cycles after dV released the slot).  Steady state, which
   // is power-limited at 950 W (S 8192, 32/8 heads, diagonal / full): 1.62 / 3.25 ms with paced vector reductions,
-  // 1.51 / 2.93 with bulk ones; 1 KB instead of 2 KB per reduction costs 4 %.
+  // 1.51 / 2.93 with bulk ones; 1 KB instead of 2 KB per reduction costs 4 %.  Head dim 256 has 17 KB left, enough for
+  // buffers of 1 KB; it keeps vector reductions, bulk ones have not been measured there.
   static constexpr bool kStageDQ = (DP <= 128);
   static constexpr int kDQGroups = (DP == 64) ? BQ / 8 : 4;      // row groups (of 4 query rows) per bulk reduction
   static constexpr int kDQBufBytes = kDQGroups * 512;            // one warp: 32 lanes x 16 bytes per row group
@@ -654,7 +653,7 @@ __global__ void __launch_bounds__(640, 1)
               float4 v = make_float4(__uint_as_float(r[4 * k + 0]) * mul, __uint_as_float(r[4 * k + 1]) * mul,
                                      __uint_as_float(r[4 * k + 2]) * mul, __uint_as_float(r[4 * k + 3]) * mul);
               if (p.reduce_out) {
-                // several CTAs (one per slice of the GQA group) add into the same rows; the host prepared dkdv_out
+                // several CTAs (one per run of the query tiles) add into the same rows; the host prepared dkdv_out
                 red_add_v4_f32(p.dkdv_out + base + c * 32 + k * 4, v.x, v.y, v.z, v.w);
               } else {
                 if (p.accumulate_prev) {
@@ -678,8 +677,8 @@ __global__ void __launch_bounds__(640, 1)
     // =========================== dQ reduction warpgroups ===========================
     // Two warpgroups, each owning half of the query columns of dQ^T.  A thread pulls its whole share into registers
     // with one batch of loads and releases the tensor-memory columns at once (the next dP^T product is waiting for
-    // them); the vector reductions into global memory, which drain at the rate the L2 can add, then overlap the next
-    // tile's products instead of sitting in front of them.
+    // them); the reductions into global memory (bulk, or vector ones at head dim 256 and in the ordered mode), which
+    // drain at the rate the L2 can add, then overlap the next tile's products instead of sitting in front of them.
     setmaxnreg_dec<80>();
     constexpr int kRedCols = BQ / 2;
     constexpr int NCR = kRedCols / 32;

@@ -492,10 +492,6 @@ template <int N>
 __device__ __forceinline__ void bulk_wait() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
-// Barrier of a subset of the block's warps (id 1..15; `threads` a multiple of 32).
-__device__ __forceinline__ void named_barrier(int id, int threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
 // Cross-CTA counters in global memory: acquire load and release add at GPU scope.
 __device__ __forceinline__ int ld_acquire_gpu(const int* gptr) {
   int v;
@@ -653,7 +649,7 @@ struct Pack2<__half> {
 
 // Optional per-role event trace (diagnostics): (tag << 48 | SM clock) records written by one
 // designated thread per role into a caller-provided buffer laid out [cta][role][cap].  Kernels are instantiated with and
-// without it: its state (spilled in part) and a test per event cost an untraced launch 4 to 10 % (backward hop of S 8192,
+// without it: its state (spilled in part) and a test per event cost an untraced launch 4 to 9 % (backward hop of S 8192,
 // 32/8 heads of 128, diagonal / full: 1.51 / 2.93 ms with, 1.38 / 2.70 without; forward full block of head dim 64 112 / 108 us).
 template <bool kOn>
 struct Tracer {
